@@ -46,7 +46,7 @@ sys.path.insert(0, ROOT)
 SEED = 2024
 N_READS = 1_000_000
 # kernels one batched call launches: dual-strand tier, second dual-strand tier (its leftovers),
-# the finishing pass, general warp tier, block tier, global tier, candidate count, scan, scatter
+# third dual-strand tier, the finishing pass, long-read tier, global tier, candidate count, scan, scatter
 LAUNCHES_PER_BATCH = 9
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_classify_dual launch on the
 # default workload (1,000,000 reads, scale 1.0): a constant from one ncu capture of this kernel,

@@ -130,8 +130,8 @@ int mg_eval_logf(mg_index* ix, const float* x, float* out, uint64_t n);
 /* Diagnostics (no counterpart in the reference). mg_set_timing(ix, 1) records CUDA events
  * around every kernel of each following classification call; mg_last_kernel_times writes the
  * last call's device times in milliseconds, 5 entries: [dual-strand warp tier with its finishing
- * pass (or the plain form's kernel), general warp tier, block tier, global-memory tier, output
- * compaction]; in the batched and served forms the second to fourth run on a second stream,
+ * pass (or the plain form's kernel), 0 (a general warp tier, now part of the next), long-read tier,
+ * global-memory tier, output compaction]; in the batched and served forms the second to fourth run on a second stream,
  * beside the finishing pass. mg_bucket_sizes returns the number of postings stored under each
  * of n 28-bit hashes (the index directory, read on the device). */
 int mg_set_timing(mg_index* ix, int on);
@@ -158,7 +158,7 @@ typedef struct {
                                   * strands mostly exceed the smaller tiers) */
   uint32_t second_blocks_per_sm; /* 4-warp blocks per SM of the 128-posting tier (1-6) */
   uint32_t finish_blocks_per_sm; /* 256-thread blocks per SM of the dual tiers' finishing pass (1-8) */
-  uint32_t long_blocks_per_sm;   /* blocks per SM of the long-read tier (1-2) */
+  uint32_t long_blocks_per_sm;   /* blocks per SM of the long-read tier (1-4) */
   uint32_t chunks;               /* pieces of a large host-buffer batch in mg_classify (1-8) */
   uint32_t weighted_chunks;      /* 1: 8 chunks weighted 1-2-3-3-3-3-2-1; 2: equal chunks */
   uint32_t third_blocks_per_sm;  /* 2-warp blocks per SM of the 256-posting tier (1-6) */
@@ -178,8 +178,9 @@ int mg_gather_bandwidth(int device, uint64_t buffer_bytes, double* gbs);
 int mg_last_kernel_times(mg_index* ix, float* ms5);
 /* Diagnostic: how many reads each tier of the last batched call run in one piece (the device
  * form, or host buffers too few to chunk) handed on: [the 64-, 128- and 256-posting dual-strand
- * tiers, the general warp tier, the smaller and the larger long-read size, the block tier] (the
- * last goes to the global-memory tier). With first_tier 2 or 3 the tiers before it count 0. */
+ * tiers, the last of these again (a general warp tier, now part of the long-read tier), the long-read
+ * tier's half-blocks and its whole block (both also count a strand that keeps every reference and was
+ * finished outside their tables), the long-read tier in all] (the last goes to the global-memory tier). With first_tier 2 or 3 the tiers before it count 0. */
 int mg_last_tier_counts(mg_index* ix, uint32_t* counts7);
 int mg_bucket_sizes(mg_index* ix, const uint32_t* hashes, uint32_t* counts, uint64_t n);
 

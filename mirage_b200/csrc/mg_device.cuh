@@ -63,12 +63,9 @@ struct BatchDev {
   uint32_t* ovf0;                // reads handed to the second dual-strand tier
   unsigned int* n_ovf0;
   unsigned int* work0b;          // cursor over ovf0
-  uint32_t* ovf0b;               // reads handed to the general warp tier
+  uint32_t* ovf0b;               // reads handed to the long-read tier
   unsigned int* n_ovf0b;
-  unsigned int* work1;           // cursor over ovf0b
-  uint32_t* ovf1;                // reads handed to the block tier
-  unsigned int* n_ovf1;
-  unsigned int* work2;           // cursor over ovf1
+  unsigned int* work2;           // cursor over ovf0b (block tier)
   uint32_t* ovf2;                // reads handed to the global-memory tier
   unsigned int* n_ovf2;
   unsigned int* work3;           // cursor over ovf2

@@ -1,5 +1,5 @@
 // mirage_b200 C ABI: index upload, the relative-score logf table, the classification kernels
-// (warp tier, block tier, global-memory tier), output compaction and the host entry points.
+// (dual-strand tiers, long-read tier, global-memory tier), output compaction and the host entry points.
 #include <cuda_runtime.h>
 
 #include <cub/device/device_scan.cuh>
@@ -49,25 +49,12 @@ int set_error(int code, const std::string& msg) {
 
 // ------------------------------------------------------------------------------ tiers
 
-// Warp tiers: one warp per read, workspace in shared memory (8 warps per block). The dual-strand
-// tier takes reads up to kLeanQ bases with at most 64 postings and 8 scored candidates per strand;
-// the general warp tier takes its leftovers within the limits below.
+// First dual-strand tier: one warp per read, 8 warps per block.
 constexpr int kW1Warps = 8;
-constexpr int kW1Q = 320, kW1Seeds = 20, kW1E = 128, kW1C = 8;
 constexpr int kW1Chunk = 4;  // reads taken per work-stealing step (default)
 
-struct WarpSmem {
-  uint64_t kA[kW1E];
-  uint32_t kB[kW1E];
-  uint32_t X[kW1E];
-  uint32_t Y[kW1E];
-  uint32_t fpos[32];
-  mg_candidate cb[2][kW1C];
-  uint8_t q[kW1Q];
-  RedTmp<32> red;
-};
-
-// Block tier: one block of 256 threads per read, workspace in dynamic shared memory.
+// Block tier: one block of 256 threads per read, workspace in dynamic shared memory; in place of the
+// long-read tier for indexes of more references than its packed postings hold (2^21).
 constexpr int kB2Threads = 256;
 constexpr int kB2Q = 20480, kB2Seeds = 1408, kB2E = 4096, kB2C = 128;
 // Global tier: one block per read, workspace in global scratch.
@@ -134,7 +121,7 @@ struct StageDev {
 };
 
 // Dual-strand warp tier: every read of the batch, one warp per read (a half-warp per strand),
-// work stealing in chunks of kW1Chunk reads; reads that do not fit go to the general warp tier.
+// work stealing in chunks of kW1Chunk reads; reads that do not fit go to the 128-posting tier.
 __global__ void __launch_bounds__(kW1Warps * 32, 5) k_classify_dual(DevIndex ix, BatchDev b, StageDev sd, uint32_t chunk) {
   __shared__ DualSmem sm[kW1Warps];
   __shared__ uint8_t comp[256];
@@ -162,62 +149,16 @@ __global__ void __launch_bounds__(kW1Warps * 32, 5) k_classify_dual(DevIndex ix,
   }
 }
 
-// Four bytes p..p+3, all readable, as one little-endian word: the aligned word holding p and,
-// only when p is not 4-aligned, the next aligned word (which holds p+3), so nothing outside
-// p..p+3's words is read.
-__device__ __forceinline__ uint32_t load4(const uint8_t* p) {
-  const uintptr_t a = (uintptr_t)p;
-  const uint32_t* w = (const uint32_t*)(a & ~(uintptr_t)3);
-  const uint32_t sh = (uint32_t)(a & 3u);
-  const uint32_t lo = w[0];
-  return sh ? __funnelshift_r(lo, w[1], sh * 8u) : lo;
-}
-// upper_dev on each byte of w: bytes 0x61..0x7F lose 0x20.
-__device__ __forceinline__ uint32_t upper4(uint32_t w) {
-  const uint32_t m = (((w & 0x7F7F7F7Fu) + 0x1F1F1F1Fu) & ~w) & 0x80808080u;
-  return w - (m >> 2);
-}
-
 constexpr int kFinThreads = 256;
 constexpr int kCovStride = kLeanQ / 32 + 1;  // coverage words per thread; odd, so no bank conflicts
 constexpr int kFinRecCap = 128;              // run records a warp walks together per 32 reads
 
-// The head and tail walks of one run record x (head_walk, tail_walk) on the strand's bases, read
-// from the batch (raw, L bytes): forward in upper case, the reverse complement backwards through
-// the complement table; the tail four bytes at a time while the window has four left. Returns the
-// run's query start << 16 | its extended length T, or 0 when T < k.
+// The walks of one run record x (process_read_dual).
 __device__ __forceinline__ uint32_t walk_record(const DevIndex& ix, const uint8_t* comp, const uint8_t* raw, uint32_t L,
                                                 int strand, const mg_candidate& x, uint32_t k, uint32_t step) {
-  auto qb = [&](uint32_t p) -> uint8_t { return strand ? comp[raw[L - 1 - p]] : upper_dev(raw[p]); };
-  const uint8_t* rs = ix.bases + ix.ref_off[x.ref];
-  const uint32_t rlen = ix.ref_len[x.ref];
-  const uint32_t sr = __float_as_uint(x.rel), lr = __float_as_uint(x.score), jj = __float_as_uint(x.pct);
-  const uint32_t sq = (jj & 0xFFu) * step, lq = (jj >> 8) * step + step;
-  uint32_t tail = 0;
-  if (lq < L && lr < rlen) {
-    const uint32_t lim = min(min(rlen - lr, k), L - lq);
-    while (tail + 4 <= lim) {
-      uint32_t wq;
-      if (strand) {
-        const uint32_t w = load4(raw + (L - 4 - (lq + tail)));
-        wq = (uint32_t)comp[w >> 24] | ((uint32_t)comp[(w >> 16) & 0xFFu] << 8) |
-             ((uint32_t)comp[(w >> 8) & 0xFFu] << 16) | ((uint32_t)comp[w & 0xFFu] << 24);
-      } else {
-        wq = upper4(load4(raw + lq + tail));
-      }
-      if (wq ^ load4(rs + lr + tail)) break;
-      tail += 4;
-    }
-    while (tail < lim && qb(lq + tail) == rs[lr + tail]) tail++;
-  }
-  uint32_t head = 0;
-  const uint32_t hsz = min(sr, k);
-  if (sq != 0 && hsz != 0) {
-    const uint32_t jb = min(sq - 1, hsz - 1);
-    while (head < jb && qb(sq - 1 - head) == rs[sr - head]) head++;
-  }
-  const uint32_t tot = tail + head + (lq - sq);
-  return tot >= k ? ((sq - head) << 16) | tot : 0u;
+  const uint32_t jj = __float_as_uint(x.pct);
+  return walk_run(ix, comp, raw, L, strand, x.ref, __float_as_uint(x.rel), __float_as_uint(x.score), (jj & 0xFFu) * step,
+                  (jj >> 8) * step + step, k);
 }
 
 // Finishing pass of the dual-strand tiers over the reads they left kReadUnscored, a warp per 32
@@ -382,58 +323,31 @@ __global__ void __launch_bounds__(Warps * 32) k_classify_dual_list(DevIndex ix, 
   }
 }
 
-// General warp tier over the dual tiers' leftovers; its own leftovers go to the block tier.
-__global__ void __launch_bounds__(kW1Warps * 32) k_classify_warp_list(DevIndex ix, BatchDev b, StageDev sd) {
-  __shared__ WarpSmem sm[kW1Warps];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  WarpSmem& S = sm[w];
-  StrandWS ws;
-  ws.q = S.q;
-  ws.fpos = S.fpos;
-  ws.kA = S.kA;
-  ws.kB = S.kB;
-  ws.X = S.X;
-  ws.Y = S.Y;
-  ws.cb[0] = S.cb[0];
-  ws.cb[1] = S.cb[1];
-  const Caps caps{kW1Q, kW1Seeds, kW1E, kW1C};
-  const uint32_t n = *b.n_ovf0b;
-  for (;;) {
-    uint32_t item = 0;
-    if (lane == 0) item = atomicAdd(b.work1, 1u);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= n) break;
-    const uint32_t r = b.ovf0b[item];
-    if (!process_read<32>(ix, b, r, ws, caps, &S.red, sd.stage, sd.arena, sd.arena_cap, sd.arena_n, b.err)) {
-      if (lane == 0) {
-        unsigned at = atomicAdd(b.n_ovf1, 1u);
-        b.ovf1[at] = r;
-      }
-    }
-    __syncwarp();
-  }
-}
-
-// Long-read tier over the general warp tier's leftovers (reads beyond its limits), a block per
-// read with work stealing: the smaller size first, then the larger over what it hands on, whose
-// own leftovers go to the block tier.
-template <class SM, int MinBlocks>
-__global__ void __launch_bounds__(kLgThreads, MinBlocks) k_classify_long(DevIndex ix, BatchDev b, StageDev sd,
-                                                                      const uint32_t* list, const unsigned* list_n,
-                                                                      unsigned* cursor, uint32_t* next,
-                                                                      unsigned* next_n) {
+// Long-read tier over the dual tiers' leftovers and the plain form's, a block per read with work
+// stealing (the next read is taken while this one is classified); its own leftovers go to the
+// global-memory tier.
+__global__ void __launch_bounds__(2 * LongSmem::H, 4) k_classify_long(DevIndex ix, BatchDev b, StageDev sd,
+                                                                     const uint32_t* list, const unsigned* list_n,
+                                                                     unsigned* cursor, uint32_t* next,
+                                                                     unsigned* next_n, unsigned* n_small,
+                                                                     unsigned* n_large) {
   extern __shared__ __align__(16) uint8_t dsm[];
-  SM& S = *reinterpret_cast<SM*>(dsm);
+  LongSmem& S = *reinterpret_cast<LongSmem*>(dsm);
   __shared__ uint32_t s_item;
   const uint32_t n = *list_n;
+  if (blockIdx.x >= n) return;
+  for (int c = threadIdx.x; c < 256; c += blockDim.x) S.comp[c] = complement_dev(upper_dev((uint8_t)c));
+  if (threadIdx.x == 0) S.handed = 0;
+  uint32_t ahead = threadIdx.x == 0 ? atomicAdd(cursor, 1u) : 0u;
   for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(cursor, 1u);
+    if (threadIdx.x == 0) s_item = ahead;
     __syncthreads();
     const uint32_t item = s_item;
-    __syncthreads();
     if (item >= n) break;
+    if (threadIdx.x == 0) ahead = atomicAdd(cursor, 1u);
     const uint32_t r = list[item];
-    if (!process_read_long(ix, b, r, S, sd.stage, sd.arena, sd.arena_cap, sd.arena_n, b.err)) {
+    if (!process_read_long(ix, b, r, S, sd.stage, sd.arena, sd.arena_cap, sd.arena_n, b.err, n_small, n_large, list,
+                           n, ahead)) {
       if (threadIdx.x == 0) next[atomicAdd(next_n, 1u)] = r;
     }
     __syncthreads();
@@ -1085,7 +999,6 @@ static int open_image(mg_index* ix, const uint8_t* image, uint64_t L, int k, int
 struct Shapes {
   unsigned dual_blocks_per_sm, steal_chunk, first_tier, second_blocks_per_sm, finish_blocks_per_sm,
       long_blocks_per_sm, chunks, weighted_chunks, third_blocks_per_sm, pack_bases;
-  unsigned long_small_blocks_per_sm;  // the smaller long-read size: its occupancy (not tuned)
 };
 
 static int occupancy(const void* fn, int threads, size_t smem) {
@@ -1095,16 +1008,12 @@ static int occupancy(const void* fn, int threads, size_t smem) {
 }
 
 static Shapes shapes(const mg_index* ix) {
-  static int occ_dual = 0, occ_second = 0, occ_third = 0, occ_long = 0, occ_long_s = 0;
+  static int occ_dual = 0, occ_second = 0, occ_third = 0, occ_long = 0;
   if (!occ_dual) {
-    cudaFuncSetAttribute(k_classify_long<LongSmem, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(LongSmem));
-    cudaFuncSetAttribute(k_classify_long<LongSmemS, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(LongSmemS));
+    cudaFuncSetAttribute(k_classify_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LongSmem));
     occ_second = occupancy((const void*)k_classify_dual_list<128, kW2Warps>, kW2Warps * 32, 0);
     occ_third = occupancy((const void*)k_classify_dual_list<256, kW3Warps>, kW3Warps * 32, 0);
-    occ_long = occupancy((const void*)k_classify_long<LongSmem, 2>, kLgThreads, sizeof(LongSmem));
-    occ_long_s = occupancy((const void*)k_classify_long<LongSmemS, 4>, kLgThreads, sizeof(LongSmemS));
+    occ_long = occupancy((const void*)k_classify_long, 2 * LongSmem::H, sizeof(LongSmem));
     occ_dual = occupancy((const void*)k_classify_dual, kW1Warps * 32, 0);
   }
   const mg_tuning& t = ix->tune;
@@ -1122,7 +1031,6 @@ static Shapes shapes(const mg_index* ix) {
   s.pack_bases = pick(t.pack_bases, 1, 1, 2);
   s.finish_blocks_per_sm = pick(t.finish_blocks_per_sm, 8, 1, 8);
   s.long_blocks_per_sm = pick(t.long_blocks_per_sm, (unsigned)occ_long, 1, (unsigned)occ_long);
-  s.long_small_blocks_per_sm = (unsigned)occ_long_s;
   s.chunks = pick(t.chunks, mg_index::kMaxChunks, 1, mg_index::kMaxChunks);
   s.weighted_chunks = pick(t.weighted_chunks, 1, 1, 2);
   return s;
@@ -1197,18 +1105,17 @@ int ensure_workspace(Workspace& w, uint64_t n_reads, uint64_t n_bases, bool host
   }
   if (w.stage.alloc(n_reads * kSlots * sizeof(mg_candidate) + 16) ||
       w.arena.alloc(arena_cap * sizeof(mg_candidate)) || w.ctr.alloc(256) ||
-      w.ovf.alloc(8 * (n_reads + 4) * 4 + 16) || w.sums.alloc(((n_reads + kScanBlock - 1) / kScanBlock + 1) * 8))
+      w.ovf.alloc(5 * (n_reads + 4) * 4 + 16) || w.sums.alloc(((n_reads + kScanBlock - 1) / kScanBlock + 1) * 8))
     return set_error(MG_ERR_OOM, "staging buffers");
   const WsLayout l3 = ws_layout(kB3Q, kB3Seeds, kB3E, kB3C);
   if (w.gws.alloc(l3.total * kB3Blocks)) return set_error(MG_ERR_OOM, "global workspace");
   return MG_OK;
 }
 
-// Counters in w_ctr (device): 0 n_cands(u64) | 8 arena_n(u64) | 16 err | 20 work | 24 n_ovf1 |
-// 28 work2 | 32 n_ovf2 | 36 work3 | 40 total(u64) | 48 n_ovf0 | 52 work1 | 56 n_ovf0b | 60 work0b |
-// 64 n_ovf1b | 68 work of the smaller long-read size | 72 n_ovf0c | 76 work0c | 80 n_ovf1c |
-// 84 work of the larger long-read size | 88 n_ovf3 (the global tier's leftovers) | 92 work4 |
-// 96 oversize need: most bases, seeds, postings, reads waiting (4 x u32)
+// Counters in w_ctr (device): 0 n_cands(u64) | 8 arena_n(u64) | 16 err | 20 work | 28 work2 |
+// 32 n_ovf2 | 36 work3 | 40 total(u64) | 48 n_ovf0 | 56 n_ovf0b | 60 work0b | 64 n_large |
+// 68 work of the long-read tier | 72 n_ovf0c | 76 work0c | 80 n_small | 88 n_ovf3 (the global tier's
+// leftovers) | 92 work4 | 96 oversize need: most bases, seeds, postings, reads waiting (4 x u32)
 int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs, const uint8_t* d_bases,
                         mg_read_result* d_reads, mg_candidate* d_out, uint64_t cap, cudaStream_t st,
                         bool plain, unsigned long long* chain, const ChainSync* cs) {
@@ -1224,28 +1131,22 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
   b.n_cands = (unsigned long long*)(ctr + 0);
   b.err = chain ? (int*)(chain + 1) : (int*)(ctr + 16);
   b.work = (unsigned*)(ctr + 20);
-  b.n_ovf1 = (unsigned*)(ctr + 24);
   b.work2 = (unsigned*)(ctr + 28);
   b.n_ovf2 = (unsigned*)(ctr + 32);
   b.work3 = (unsigned*)(ctr + 36);
   b.n_ovf0 = (unsigned*)(ctr + 48);
-  b.work1 = (unsigned*)(ctr + 52);
   b.n_ovf0b = (unsigned*)(ctr + 56);
   b.work0b = (unsigned*)(ctr + 60);
   b.ovf0 = w.ovf.as<uint32_t>();
   b.ovf0b = w.ovf.as<uint32_t>() + 3 * (n + 4);
-  b.ovf1 = w.ovf.as<uint32_t>() + n + 4;
   b.ovf2 = w.ovf.as<uint32_t>() + 2 * (n + 4);
-  uint32_t* ovf1b = w.ovf.as<uint32_t>() + 4 * (n + 4);  // the long-read tier's leftovers
-  unsigned* n_ovf1b = (unsigned*)(ctr + 64);
+  unsigned* n_large = (unsigned*)(ctr + 64);  // reads that the long-read tier's whole block could not take
   unsigned* work_long = (unsigned*)(ctr + 68);
-  uint32_t* ovf0c = w.ovf.as<uint32_t>() + 5 * (n + 4);  // the 128-posting tier's leftovers
+  uint32_t* ovf0c = w.ovf.as<uint32_t>() + n + 4;  // the 128-posting tier's leftovers
   unsigned* n_ovf0c = (unsigned*)(ctr + 72);
   unsigned* work0c = (unsigned*)(ctr + 76);
-  uint32_t* ovf1c = w.ovf.as<uint32_t>() + 6 * (n + 4);  // the smaller long-read size's leftovers
-  unsigned* n_ovf1c = (unsigned*)(ctr + 80);
-  unsigned* work_long2 = (unsigned*)(ctr + 84);
-  uint32_t* ovf3 = w.ovf.as<uint32_t>() + 7 * (n + 4);  // the global tier's leftovers
+  unsigned* n_small = (unsigned*)(ctr + 80);  // reads that its half-blocks could not take
+  uint32_t* ovf3 = w.ovf.as<uint32_t>() + 4 * (n + 4);  // the global tier's leftovers
   unsigned* n_ovf3 = (unsigned*)(ctr + 88);
   unsigned* work4 = (unsigned*)(ctr + 92);
   unsigned* huge_need = (unsigned*)(ctr + 96);
@@ -1264,16 +1165,13 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
   static bool attr_set = false;
   if (!attr_set) {
     CU(cudaFuncSetAttribute(k_classify_block<kB2Threads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l2.total));
-    CU(cudaFuncSetAttribute(k_classify_long<LongSmem, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)sizeof(LongSmem)));
-    CU(cudaFuncSetAttribute(k_classify_long<LongSmemS, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)sizeof(LongSmemS)));
+    CU(cudaFuncSetAttribute(k_classify_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LongSmem)));
     attr_set = true;
   }
   const bool tm = ix->timing && ix->events_made;
   if (n > 0) {
-    // timing events (start, end) per tier: ev[0..1] first tier, ev[2..3] general warp tier,
-    // ev[3..4] block tier, ev[4..5] global tier, ev[6..7] compaction
+    // timing events (start, end) per tier: ev[0..1] first tier, ev[2..3] nothing,
+    // ev[3..4] long-read tier, ev[4..5] global tier, ev[6..7] compaction
     if (tm) CU(cudaEventRecord(ix->ev[0], st));
     auto global_tier = [&](cudaStream_t s) {
       k_classify_block<kB3Threads><<<kB3Blocks, kB3Threads, 0, s>>>(ix->dix, b, sd, b.ovf2, b.n_ovf2, b.work3, ovf3,
@@ -1316,16 +1214,13 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
       CU(cudaEventRecord(w.fork, st));
       CU(cudaStreamWaitEvent(w.side, w.fork, 0));
       if (tm) CU(cudaEventRecord(ix->ev[2], w.side));
-      static int per_sm2 = 0;  // the same on every call (one architecture): queried once
-      if (!per_sm2) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_classify_warp_list, kW1Warps * 32, 0);
-      k_classify_warp_list<<<(unsigned)std::max(1, per_sm2) * sms, kW1Warps * 32, 0, w.side>>>(ix->dix, b, sd);
       if (tm) CU(cudaEventRecord(ix->ev[3], w.side));
-      k_classify_long<LongSmemS, 4><<<sh.long_small_blocks_per_sm * sms, kLgThreads, sizeof(LongSmemS), w.side>>>(
-          ix->dix, b, sd, b.ovf1, b.n_ovf1, work_long, ovf1c, n_ovf1c);
-      k_classify_long<LongSmem, 2><<<sh.long_blocks_per_sm * sms, kLgThreads, sizeof(LongSmem), w.side>>>(
-          ix->dix, b, sd, ovf1c, n_ovf1c, work_long2, ovf1b, n_ovf1b);
-      k_classify_block<kB2Threads><<<(unsigned)sms, kB2Threads, l2.total, w.side>>>(
-          ix->dix, b, sd, ovf1b, n_ovf1b, b.work2, b.ovf2, b.n_ovf2, nullptr, l2, c2, 0);
+      if (ix->dix.n_refs <= (1u << 21))
+        k_classify_long<<<sh.long_blocks_per_sm * sms, 2 * LongSmem::H, sizeof(LongSmem), w.side>>>(
+            ix->dix, b, sd, b.ovf0b, b.n_ovf0b, work_long, b.ovf2, b.n_ovf2, n_small, n_large);
+      else
+        k_classify_block<kB2Threads><<<(unsigned)sms, kB2Threads, l2.total, w.side>>>(
+            ix->dix, b, sd, b.ovf0b, b.n_ovf0b, b.work2, b.ovf2, b.n_ovf2, nullptr, l2, c2, 0);
       if (tm) CU(cudaEventRecord(ix->ev[4], w.side));
       global_tier(w.side);
       if (tm) CU(cudaEventRecord(ix->ev[5], w.side));
@@ -1894,9 +1789,10 @@ int mg_last_tier_counts(mg_index* ix, uint32_t* counts7) {
   uint8_t h[128];
   CU(cudaStreamSynchronize(ix->stream));
   CU(cudaMemcpy(h, ix->ws.ctr.p, sizeof(h), cudaMemcpyDeviceToHost));
-  // the lists' counters (run_pipeline): left by the 64-, 128- and 256-posting dual tiers, the
-  // general warp tier, the two long-read sizes and the block tier
-  static const int at[7] = {48, 72, 56, 24, 80, 64, 32};
+  // the lists' counters (run_pipeline): left by the 64-, 128- and 256-posting dual tiers (the last
+  // also as the general warp tier's entry, which has no tier of its own any more), by the long-read
+  // tier's half-blocks and its whole block, and in all for the global-memory tier
+  static const int at[7] = {48, 72, 56, 56, 80, 64, 32};
   for (int i = 0; i < 7; i++) std::memcpy(&counts7[i], h + at[i], 4);
   return MG_OK;
 }

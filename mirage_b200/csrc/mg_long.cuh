@@ -1,173 +1,418 @@
-// Long-read tier: reads longer than the warp tiers take, one block of kLgThreads threads per
-// read, both strands in turn, over reads taken from a list by work stealing. Two sizes: reads up
-// to kLsQ bases with up to kLsE postings and kLsK kept postings per strand in a block of about
-// 51 KB of shared memory (four blocks per SM), then what they hand on, up to kLgQ bases, kLgE
-// postings and kLgK kept postings, in blocks of about 105 KB (two per SM).
+// Group form of the classification: reads that the dual-strand warp tiers do not take (over kLeanQ
+// bases, or more postings than they hold) and every read of the plain form. A block takes a read;
+// its two halves of H threads take one strand each, side by side, and synchronise on a named
+// barrier each; a strand that does not fit its half's share of the shared memory makes the whole
+// block take the strands in turn with all of it. What does not fit then goes to the next tier.
 //
-// The general path (process_strand, mg_kernels.cuh) sorts every posting of a strand twice:
-// by (refID, found index) for the occurrence filter and again, with the postings it dropped
-// padded in, by (refID, position, query position) for the diagonal runs. A 5 kb read has about
-// 750 postings per strand, a 20 kb read 3,000, while only the postings of the one or two
-// references with the longest occurrence runs survive the filter. Here the filter needs no sort:
-//   occurrence filter  every (refID, found index) pair of the strand goes into a hash set in
-//                      shared memory; a pair whose (refID, found index - 1) is absent starts an
-//                      occurrence run, whose length is the number of (refID, found index + t)
-//                      present after it; occMax of a reference is its longest run
-//                      (Analyser.cpp:2057-2115: consecutive found indices of one reference, a
-//                      reference counted once per found index), hs the longest of all
-//   keep rule          the references with a run of at least max(1, hs - 1) go to a small table
-//                      and only their postings are compacted (Analyser.cpp:2115-2196)
-//   sort               the kept postings only, by (refID, position, query position)
-// and the diagonal runs, the walks, the coverage and the scores follow as in process_strand
-// (Analyser.cpp:2337-2490, MatrixCPU.cpp:18-214), the coverage through a bitmap in shared memory.
+// The strand's bases are hashed from global memory (a seed's window is five aligned words), so
+// shared memory holds postings only, 8 bytes each plus a 2-byte index, in seed order.
+//   links              a posting is linked when its reference also has a posting under the found seed
+//                      before its own (found indices f and f - 1, Analyser.cpp:2057-2115). A reference
+//                      with no linked posting has no occurrence run of 2 and so no diagonal run of 2
+//                      (one diagonal, consecutive seeds), which a candidate needs (:2402): only
+//                      references with a link matter, and a strand without any is done. The search
+//                      goes through the previous seed's bucket from just before the posting's own
+//                      place in its bucket: copies of a repeat keep their order from bucket to bucket,
+//                      so they meet in a few comparisons; buckets of random hits are one or two long.
+//   occurrence filter  per linked reference a bitmap of the found indices where it occurs; its longest
+//                      run of ones is occMax; references with max(2, hs - 1) or more stay (:2115)
+//   order              the kept postings by reference, each one's in seed order (a posting's place is
+//                      the number of ones before its found index in the bitmap): that is (position,
+//                      seed) order unless a stray hit interferes, which is checked; then each
+//                      reference's postings are ranked by a warp, or, when one has more than kRankMax,
+//                      sorted by the block
+//   runs, walks        run starts as a bit mask; a run's length reaches back to the last start
+//                      (:2337-2490); a thread walks a run end's head and tail and adds its length,
+//                      triangle and covered bases to its reference's sums and bitmap (MatrixCPU.cpp:18-214)
+//
+// What bounds it: latency, of the slots' DRAM pages and of some twenty group-wide steps a strand, with
+// eight strands in flight per SM (issue slots 27% used, DRAM 1.3 TB/s). Measured on a B200 against the
+// form before it (two sizes of block, one strand at a time on 256 threads, a hash set of (refID, found
+// index) pairs, then a block per SM with two full sorts for what they left): 20,000 reads of 1-20 kb
+// on 5,000 references 5.86 -> 1.87 ms, 200,000 reads of 250 bases on references sharing repeats (36
+// copies of a segment) 4.50 -> 2.19 ms, 4,001 reads of 75 bases to 20 kb from host memory 1.28 -> 0.70 ms.
 #pragma once
-#include "mg_kernels.cuh"
+#include "mg_lean.cuh"
 
 namespace mg {
 
-constexpr int kLgThreads = 256;
-constexpr int kLgQ = 20480;     // longest read (the config's 20 kb reads)
-constexpr int kLgSeeds = 2047;  // seeds per strand (found index and seed index take 11 bits each)
-constexpr int kLgE = 4096;      // postings per strand
-constexpr int kLsQ = 8192;      // the smaller size: longest read
-constexpr int kLsE = 2048;      // the smaller size: postings per strand
-constexpr int kLgK = 2048;      // kept postings per strand (the larger size)
-constexpr int kLsK = 1024;      // the smaller size: kept postings per strand
-constexpr int kLgC = 64;        // scored candidates per strand
-constexpr int kLgRT = 128;      // table of kept references (at most half of it used)
 constexpr uint32_t kLgEmpty = 0xFFFFFFFFu;
+constexpr uint32_t kLgKeepAll = 64;       // see long_strand's `wide`
+constexpr uint32_t kRankMax = 128;        // postings of a reference that a warp ranks
+constexpr uint32_t kLgWork = 1u << 21;    // most comparisons of the link search (sum of squared buckets)
 
-// Dynamic shared memory of one block. From the compaction on, the hash set holds the sort keys
-// (kA: K uint64, kB: K uint32), p_ref and p_pos the per-entry scratch X and Y, and p_fj
-// the coverage bitmap.
-template <int Q, int E, int K>
-struct alignas(16) LongSmemT {
-  static constexpr int kQ = Q, kE = E, kK = K;
-  uint32_t hs[2 * E];         // (refID << 11 | found index) set, open addressing
-  uint32_t p_ref[E];          // the strand's postings in seed order
-  uint32_t p_pos[E];
-  uint32_t p_fj[E];           // found index | seed index << 11 | 1 << 31 for the pair's first posting
-  uint32_t rt[kLgRT];         // kept references
-  mg_candidate cb[2][kLgC];   // scored candidates of the two strands
-  RedTmp<kLgThreads> red;
-  uint32_t n_kept, n_rt;
-  uint32_t scored[kLgC / 32];  // candidates with a score (bit per candidate)
-  uint32_t rrank[kLgRT];       // kept reference of a table slot: its rank by refID
-  uint32_t bcnt[kLgRT / 2], bfill[kLgRT / 2], boff[kLgRT / 2 + 1], bmax;  // the kept references' ranges
-  uint32_t n_sc;
-  float hi;
-  uint8_t q[Q];               // strand bases
-  static_assert(K * 12 <= 2 * E * 4 && K <= E && Q / 32 + 1 <= E && 4 * kLgThreads <= 2 * E, "aliased regions");
+// Shared memory of a block: two halves of H threads, each with room for E postings, NS seeds and RM
+// kept references per strand (RT table slots); the whole block uses both shares of the postings and
+// seeds for one strand.
+template <int H_, int E_, int NS_, int RT_, int RM_>
+struct alignas(16) LongSm {
+  static constexpr int H = H_, E = E_, NS = NS_, RT = RT_, RM = RM_;
+  static constexpr int NSP = NS + 1, NW = (NS + 31) / 32, BW = E / 64;  // BW: words of E / 2 bits
+  struct Half {
+    unsigned long long sumr[RM];  // sums of a candidate's runs; before: the linked references' best
+    uint32_t sumc[RM];            // runs (sumr), their refIDs (sumc), the ranges' bounds
+    uint32_t segmax[RM];          // longest diagonal run of a kept reference; then its covered bases
+    uint32_t kref[RM];            // kept references by refID
+    uint32_t rt[RT];              // table of linked references
+    uint8_t rid[RT];              // a slot's reference: order of insertion
+    uint16_t cnt[RM];             // kept postings (by order of insertion)
+    uint8_t rk[RM], kid[RM];      // rank among the kept references (kNoId: none) by order of insertion, and back
+  };
+  uint32_t rs[2 * E];  // refID << 11 | seed
+  uint32_t ps[2 * E];  // reference position
+  // per share: sorted order (E / 2), kept postings (E / 2), first posting of each seed (NSP); the
+  // seeds' hashes and then the linked references' bitmaps lie over the first two, the candidates'
+  // coverage over the last
+  uint16_t pool[2 * (E + NSP)];
+  uint32_t fm[2 * NW];  // found seeds
+  uint16_t fp[2 * NW];  // found seeds before each word of fm
+  uint32_t bk[2 * BW];  // starts of diagonal runs
+  uint32_t red[2][2][2 * H / 32];
+  uint32_t n_rt[2], over[2], dup[2], n_ends[2], n_out[2], handed;
+  float hi[2];
+  int status[2];
+  uint32_t cand_at, ahead;
+  Half h[2];
+  mg_candidate cb[2][RM];
+  uint8_t comp[256];  // complement(upper(byte)), 0 where there is none
+  static_assert(E % 64 == 0 && (E + NSP) % 4 == 0 && NSP % 2 == 0 && 2 * E <= 8192 && NS <= E / 2 && 2 * NS <= 2047 && RT <= 256 && RM < 127, "sizes");
+  static_assert(RM * 8 >= 2 * (RM + 1), "tables over the sums");
 };
-using LongSmem = LongSmemT<kLgQ, kLgE, kLgK>;   // two blocks per SM
-using LongSmemS = LongSmemT<kLsQ, kLsE, kLsK>;  // four blocks per SM
-static_assert(2 * (sizeof(LongSmem) + 1024) <= 233472, "two blocks per SM");
-static_assert(4 * (sizeof(LongSmemS) + 1024) <= 233472, "four blocks per SM");
+
+// The classes of reads: the batched forms' tier (reads to 20,480 bases and 4,096 postings per strand)
+// with four blocks per SM, and the plain form's first kernel, one block of two warps per read.
+using LongSmem = LongSm<128, 2048, 1023, 256, 96>;
+constexpr uint32_t kLgQ = 20480;
+static_assert(4 * (sizeof(LongSmem) + 1024) <= 233472, "four blocks per SM");
 
 __device__ __forceinline__ uint32_t lg_mix(uint32_t x) { return (x * 2654435761u) ^ (x >> 15); }
 
-// The probes visit each slot at most once: every caller keeps its table at most half full, so an
-// empty slot ends them first; reaching the bound sets kErrInternal in *err.
-__device__ __forceinline__ bool lg_contains(const uint32_t* set, uint32_t mask, uint32_t key, int* err) {
-  uint32_t s = lg_mix(key) & mask;
-  for (uint32_t n = 0; n <= mask; n++, s = (s + 1) & mask) {
-    const uint32_t v = set[s];
-    if (v == key) return true;
-    if (v == kLgEmpty) return false;
-  }
-  *err |= kErrInternal;
-  return false;
+// Barrier over the G threads of a group (a named barrier: 1 + half for a half, 0 for the block).
+__device__ __forceinline__ void lg_sync(int bar, uint32_t G) {
+  asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(G) : "memory");
 }
 
-// The slot holding key, or -1 (bounded like lg_contains).
-__device__ __forceinline__ int lg_find(const uint32_t* set, uint32_t mask, uint32_t key, int* err) {
-  uint32_t s = lg_mix(key) & mask;
-  for (uint32_t n = 0; n <= mask; n++, s = (s + 1) & mask) {
-    const uint32_t v = set[s];
-    if (v == key) return (int)s;
-    if (v == kLgEmpty) return -1;
+// upper_dev on each byte of w: bytes 0x61..0x7F lose 0x20.
+__device__ __forceinline__ uint32_t upper4(uint32_t w) {
+  const uint32_t m = (((w & 0x7F7F7F7Fu) + 0x1F1F1F1Fu) & ~w) & 0x80808080u;
+  return w - (m >> 2);
+}
+// Whether all four bytes of w (upper case) are in ACGT: two bits of a byte pick the letter that it
+// has to be.
+__device__ __forceinline__ bool acgt4(uint32_t w) {
+  const uint32_t c = (w >> 1) & 0x03030303u;  // A 0, C 1, T 2, G 3
+  const uint32_t t = c | (c >> 4);
+  return __byte_perm(0x47544341u, 0, (t & 0xFFu) | ((t >> 8) & 0xFF00u)) == w;
+}
+// Complement of four ACGT bytes: A and T differ in 0x15, C and G (bit 1 set) in 0x04.
+__device__ __forceinline__ uint32_t comp4(uint32_t w) { return w ^ 0x15151515u ^ (((w >> 1) & 0x01010101u) * 0x11u); }
+
+// hash28_dev of the 17-byte window a..a+16 of an ACGT read in upper case (strand 0), or of its
+// reverse complement (strand 1). The five aligned words loaded each hold a byte of the window
+// ((a & 3) + 17 <= 20).
+__device__ __forceinline__ uint32_t hash17_acgt(const uint8_t* a, int strand) {
+  const uint32_t* w = (const uint32_t*)((uintptr_t)a & ~(uintptr_t)3);
+  const uint32_t sh = ((uint32_t)(uintptr_t)a & 3u) * 8u;
+  const uint32_t x0 = __ldg(w), x1 = __ldg(w + 1), x2 = __ldg(w + 2), x3 = __ldg(w + 3), x4 = __ldg(w + 4);
+  uint32_t y[5] = {__funnelshift_r(x0, x1, sh), __funnelshift_r(x1, x2, sh), __funnelshift_r(x2, x3, sh),
+                   __funnelshift_r(x3, x4, sh), x4 >> sh};
+#pragma unroll
+  for (int i = 0; i < 5; i++) y[i] = upper4(y[i]);
+  uint32_t h = 2166136261u;
+  if (strand == 0) {
+#pragma unroll
+    for (int i = 0; i < 17; i++) h = (h * 16777619u) ^ ((y[i >> 2] >> (8 * (i & 3))) & 0xFFu);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 5; i++) y[i] = comp4(y[i]);
+#pragma unroll
+    for (int i = 16; i >= 0; i--) h = (h * 16777619u) ^ ((y[i >> 2] >> (8 * (i & 3))) & 0xFFu);
   }
-  *err |= kErrInternal;
-  return -1;
+  return ((h >> 28) ^ h) & 0x0FFFFFFFu;
 }
 
-// Inserts key; true when this call inserted it (false: it was there already).
-__device__ __forceinline__ bool lg_insert(uint32_t* set, uint32_t mask, uint32_t key, int* err) {
-  uint32_t s = lg_mix(key) & mask;
-  for (uint32_t n = 0; n <= mask; n++, s = (s + 1) & mask) {
-    const uint32_t old = atomicCAS(&set[s], kLgEmpty, key);
-    if (old == kLgEmpty) return true;
-    if (old == key) return false;
-  }
-  *err |= kErrInternal;
-  return false;
+// n (1 to 8) bytes p..p+n-1 as a little-endian number, zeros above; only aligned words that hold one
+// of them are read.
+__device__ __forceinline__ uint64_t load_bytes(const uint8_t* p, uint32_t n) {
+  const uintptr_t a = (uintptr_t)p;
+  const uint32_t* w = (const uint32_t*)(a & ~(uintptr_t)3);
+  const uint32_t o = (uint32_t)(a & 3u), e = o + n;
+  const uint32_t w0 = w[0], w1 = e > 4 ? w[1] : 0u, w2 = e > 8 ? w[2] : 0u;
+  const uint64_t v = ((uint64_t)__funnelshift_r(w1, w2, 8 * o) << 32) | __funnelshift_r(w0, w1, 8 * o);
+  return v & (~0ull >> (64 - 8 * n));
+}
+// complement(upper(byte)) of four bytes, by table for those outside ACGT.
+__device__ __forceinline__ uint32_t comp_any4(uint32_t w, const uint8_t* comp) {
+  const uint32_t u = upper4(w);
+  if (acgt4(u)) return comp4(u);
+  return (uint32_t)comp[u & 0xFFu] | ((uint32_t)comp[(u >> 8) & 0xFFu] << 8) |
+         ((uint32_t)comp[(u >> 16) & 0xFFu] << 16) | ((uint32_t)comp[u >> 24] << 24);
 }
 
-// One strand of a read (raw bytes, L <= SM::kQ) on the whole block. Same contract as
-// process_strand: kStrandOverflow hands the read to the block tier.
+// The head and tail walks of a run (head_walk, tail_walk) on the strand's bases, read from the batch
+// (raw, L bytes; the reverse complement backwards, through the complement table). The run: reference
+// position of its first seed sr and reference end of its last seed lr, first query base sq and query
+// end lq. Returns the run's query start << 16 | its extended length T, or 0 when T < k.
+// Both walks advance eight bytes per round trip to memory, with the loads of a step (query and
+// reference, head and tail) in flight together: most walks end in the first or second step, and a
+// step's cost is the reference's DRAM latency, once for both. Sixteen bytes a step cost more in
+// registers and instructions than the round trips they save (the finishing pass of 1 M reads of
+// 75-300 bases: 278 us, against 226 us at eight).
+__device__ __forceinline__ uint32_t walk_run(const DevIndex& ix, const uint8_t* comp, const uint8_t* raw, uint32_t L,
+                                             int strand, uint32_t ref, uint32_t sr, uint32_t lr, uint32_t sq,
+                                             uint32_t lq, uint32_t k) {
+  const uint8_t* rs = ix.bases + ix.ref_off[ref];
+  const uint32_t rlen = ix.ref_len[ref];
+  // strand bases p..p+n-1 (1 <= n <= 8) as a number, base p in the low byte
+  auto query = [&](uint32_t p, uint32_t n) -> uint64_t {
+    if (!strand) {
+      const uint64_t v = load_bytes(raw + p, n);
+      return ((uint64_t)upper4((uint32_t)(v >> 32)) << 32) | upper4((uint32_t)v);
+    }
+    const uint64_t v = load_bytes(raw + (L - p - n), n);  // base p is the last byte of these
+    const uint32_t lo = __byte_perm((uint32_t)v, 0, 0x0123), hi = __byte_perm((uint32_t)(v >> 32), 0, 0x0123);
+    const uint64_t m = (((uint64_t)lo << 32) | hi) >> (64 - 8 * n);
+    // zeros above base p+n-1 map to the table's entry of 0: zero, as on the reference's side
+    return ((uint64_t)comp_any4((uint32_t)(m >> 32), comp) << 32) | comp_any4((uint32_t)m, comp);
+  };
+  const uint32_t tl = lq < L && lr < rlen ? min(min(rlen - lr, k), L - lq) : 0u;  // most that the tail takes
+  const uint32_t hz = min(sr, k);
+  const uint32_t hl = sq != 0 && hz != 0 ? min(sq - 1, hz - 1) : 0u;  // most that the head takes
+  uint32_t tail = 0, head = 0;
+  bool t_on = tl > 0, h_on = hl > 0;
+#pragma unroll 1
+  while (t_on || h_on) {  // a walk that goes on takes at least one base
+    const uint32_t tn = t_on ? min(8u, tl - tail) : 0u, hn = h_on ? min(8u, hl - head) : 0u;
+    uint64_t tq = 0, tr = 0, hq = 0, hr = 0;
+    if (tn) tr = load_bytes(rs + lr + tail, tn);
+    if (hn) hr = load_bytes(rs + (sr - head - hn + 1), hn);
+    if (tn) tq = query(lq + tail, tn);
+    if (hn) hq = query(sq - head - hn, hn);
+    if (tn) {
+      const uint64_t d = tq ^ tr;
+      const uint32_t same = d ? (uint32_t)(__ffsll((long long)d) - 1) >> 3 : tn;
+      tail += same;
+      t_on = same == tn && tail < tl;
+    }
+    if (hn) {
+      const uint64_t d = (hq ^ hr) << (64 - 8 * hn);  // the walk goes down from the last byte
+      const uint32_t same = d ? (uint32_t)__clzll((long long)d) >> 3 : hn;
+      head += same;
+      h_on = same == hn && head < hl;
+    }
+  }
+  const uint32_t tot = tail + head + (lq - sq);
+  return tot >= k ? ((sq - head) << 16) | tot : 0u;
+}
+
+// Longest run of ones of a bitmap of nw words (nw <= 64), on a warp; every lane gets it. before[w]
+// receives the number of ones in the words before w, *total that of all.
+__device__ __forceinline__ uint32_t warp_longest_run(const uint32_t* bm, uint32_t nw, uint16_t* before, uint32_t* total) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t n0 = 2 * lane < nw ? __popc(bm[2 * lane]) : 0u, n1 = 2 * lane + 1 < nw ? __popc(bm[2 * lane + 1]) : 0u;
+  uint32_t x = n0 + n1;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  if (2 * lane < nw) before[2 * lane] = (uint16_t)(x - n0 - n1);
+  if (2 * lane + 1 < nw) before[2 * lane + 1] = (uint16_t)(x - n1);
+  *total = __shfl_sync(0xffffffffu, x, 31);
+  // a span's (bits, leading ones, trailing ones, longest run); two words a lane, then lanes combined
+  uint32_t len = 0, pre = 0, suf = 0, best = 0;
+  auto join = [&](uint32_t l2, uint32_t p2, uint32_t s2, uint32_t b2) {  // this span, then the other
+    best = max(max(best, b2), suf + p2);
+    pre = pre == len ? len + p2 : pre;
+    suf = s2 == l2 ? l2 + suf : s2;
+    len += l2;
+  };
+#pragma unroll
+  for (uint32_t u = 0; u < 2; u++) {
+    const uint32_t w = 2 * lane + u;
+    if (w < nw) {
+      const uint32_t m = bm[w];
+      join(32, (uint32_t)__ffs(~m) ? (uint32_t)__ffs(~m) - 1u : 32u, (uint32_t)__clz(~m), (uint32_t)longest_run(m));
+    }
+  }
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t l2 = __shfl_down_sync(0xffffffffu, len, o), p2 = __shfl_down_sync(0xffffffffu, pre, o);
+    const uint32_t s2 = __shfl_down_sync(0xffffffffu, suf, o), b2 = __shfl_down_sync(0xffffffffu, best, o);
+    if (lane + o < 32) join(l2, p2, s2, b2);
+  }
+  return __shfl_sync(0xffffffffu, best, 0);
+}
+
+// One strand of a read (raw bytes, L of them, no byte without a complement; acgt: all of them letters
+// of ACGT in either case) on G threads with room for kE postings and kNS seeds: half `half` of the
+// block (G = H), or all of it (whole: G = 2 H, half 0). On kStrandOk the strand's *n_out scored candidates
+// are in cb, in ascending refID, and *highest is its HighestScore. kStrandOverflow: it does not fit.
+// *wide: the keep rule keeps more references than a table of kLgKeepAll postings' worth (hs = 2
+// keeps every reference with a posting) and the strand has a diagonal run.
+// One instance for both, and loops kept rolled: the code runs through once per strand, so that its
+// size is paid in instruction fetches. With an instance each and the compiler's unrolling it was
+// 355 KB, and four blocks per SM slowed each other from 64,000 to 119,000 cycles a read (20,000 reads
+// of 1-20 kb: 2.25 ms); at 98 KB, from 64,000 to 84,000 (1.75 ms).
 template <class SM>
-__device__ int long_strand(const DevIndex& ix, const uint8_t* raw, uint32_t L, int strand, SM& S, int* err,
-                           uint32_t* n_out, float* highest) {
-  constexpr int kE = SM::kE;
-  constexpr int G = kLgThreads;
-  const int tid = threadIdx.x;
+__device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* raw, uint32_t L, int strand, bool acgt,
+                                           SM& S, bool whole, int half, mg_candidate* cb, int* err, uint32_t* n_out,
+                                           float* highest, bool* wide) {
+  constexpr uint32_t kRT = SM::RT, kRM = SM::RM;
+  constexpr unsigned FULL = 0xffffffffu;
+  const uint32_t sh = whole ? 1u : 0u;  // twice the threads and the room
+  const uint32_t G = SM::H << sh, kE = SM::E << sh, kNS = SM::NS << sh, kNW = SM::NW << sh, kW = G / 32;
+  const int bar = whole ? 0 : 1 + half;
+  const uint32_t tid = whole ? threadIdx.x : threadIdx.x - half * SM::H;
+  const uint32_t lane = tid & 31u, warp = tid >> 5;
   const uint32_t k = (uint32_t)ix.k, step = (uint32_t)ix.step;
-  RedTmp<G>* red = &S.red;
+  uint32_t* rs = S.rs + half * SM::E;
+  uint32_t* ps = S.ps + half * SM::E;
+  uint16_t* sx = S.pool + half * (SM::E + SM::NSP);  // sorted order of the kept postings
+  uint16_t* kl = sx + kE / 2;                        // the kept postings
+  uint16_t* st = sx + kE;                            // first posting of each seed (kNS + 1)
+  uint32_t* fm = S.fm + half * SM::NW;
+  uint16_t* fp = S.fp + half * SM::NW;
+  uint32_t* bk = S.bk + half * SM::BW;
+  typename SM::Half& T = S.h[half];
+  uint32_t* iref = T.sumc;                                      // linked references in order of insertion
+  uint16_t* best = reinterpret_cast<uint16_t*>(T.sumr);         // their longest occurrence runs
+  uint16_t* boff = reinterpret_cast<uint16_t*>(T.sumr);         // then: the kept references' ranges
+  uint32_t* bfill = T.sumc;                                     // (counts, then fill)
+  uint32_t(*red)[2 * SM::H / 32] = S.red[half];
   *n_out = 0;
   *highest = -1.0f;
-  // strand bases (A0)
-  uint32_t bad = 0;
-  for (uint32_t i = tid; i < L; i += G) {
-    uint8_t c;
-    if (strand == 0) {
-      c = upper_dev(raw[i]);
-    } else {
-      c = complement_dev(upper_dev(raw[L - 1 - i]));
-      if (!c) bad = 1;
-    }
-    S.q[i] = c;
-  }
-  if (grp_max_u64<G>(bad, red)) return kStrandBad;
   if (L <= k) return kStrandOk;
   const uint32_t ns = (L - k + step - 1) / step;
-  if (ns > (uint32_t)kLgSeeds) return kStrandOverflow;
-  // 1. seeds, probe, found indices, postings in seed order
-  uint32_t nf = 0, ne = 0;
-  for (uint32_t j0 = 0; j0 < ns; j0 += G) {
-    const uint32_t j = j0 + tid;
-    uint32_t found = 0, cnt = 0, o0 = 0;
-    uint4 v0 = make_uint4(0u, 0u, 0u, 0u), v1 = v0, v2 = v0, v3 = v0;
-    if (j < ns) {
-      const uint32_t h = hash28_dev(S.q + j * step, ix.hlen);
-      if (ix.slots) {
-        const uint4* sl = ix.slots + (size_t)h * kSlotVecs;
-        v0 = __ldg(sl);
-        v1 = __ldg(sl + 1);
-        cnt = v0.x;
-        o0 = v0.y;
-        if (cnt > 3) {
-          v2 = __ldg(sl + 2);
-          v3 = __ldg(sl + 3);
-        }
-      } else {
-        o0 = __ldg(ix.dir + h);
-        cnt = __ldg(ix.dir + h + 1) - o0;
+  const uint32_t kCovWords = (SM::NSP << sh) / 2;  // over st
+  if (ns > kNS || (L + 31) / 32 > kCovWords) return kStrandOverflow;
+#pragma unroll 1
+  for (uint32_t i = tid; i < kRT; i += G) T.rt[i] = kLgEmpty;
+  if (tid == 0) {
+    S.n_rt[half] = 0;
+    S.over[half] = 0;
+  }
+  // 1. seeds, probe, postings in seed order: every seed's hash first, its slot (or directory entry)
+  //    asked for as it is known; then the bucket sizes, so that the DRAM latency is paid once for all
+  //    seeds and not once per G of them; their prefix sum; then the postings, from L2
+  uint32_t* hb = reinterpret_cast<uint32_t*>(sx);  // the seeds' hashes, over the order arrays
+#pragma unroll 1
+  for (uint32_t j = tid; j < ns; j += G) {
+    const uint32_t p = j * step;
+    uint32_t h;
+    if (acgt && ix.hlen == 17) {
+      h = hash17_acgt(raw + (strand ? L - 17 - p : p), strand);
+    } else {
+      h = 2166136261u;
+#pragma unroll 1
+      for (int t = 0; t < ix.hlen; t++) {
+        const uint8_t c = strand ? S.comp[raw[L - 1 - p - t]] : upper_dev(raw[p + t]);
+        h = (h * 16777619u) ^ c;
       }
-      found = (cnt > 0 || h == ix.empty_hash) ? 1u : 0u;
+      h = ((h >> 28) ^ h) & 0x0FFFFFFFu;
     }
-    const uint32_t x = cnt > (uint32_t)kE ? (uint32_t)kE + 1 : cnt;
-    uint32_t fr, er;
-    const uint32_t fi = grp_excl_sum<G>(found, red, &fr);
-    const uint32_t ei = grp_excl_sum<G>(x, red, &er);
-    if (ne + er > (uint32_t)kE) return kStrandOverflow;  // group-uniform
-    const uint32_t e = ne + ei, fj = (nf + fi) | (j << 11);
-    uint32_t t0 = 0;
-    if (ix.slots) {
+    hb[j] = h;
+    if (ix.slots)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(ix.slots + (size_t)h * kSlotVecs));
+    else
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(ix.dir + h));
+  }
+  const uint32_t t0 = ix.slots ? (uint32_t)kSlotPosts : 0u;  // postings of a seed from its slot
+  uint32_t sq2 = 0;   // this thread's seeds' squared bucket sizes
+  bool more = false;  // postings past a slot's
+#pragma unroll 1
+  for (uint32_t j0 = 0; j0 < ns; j0 += 4 * G) {
+    uint32_t c[4];
+    bool found[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {  // four loads in flight
+      const uint32_t j = j0 + u * G + tid;
+      c[u] = 0;
+      found[u] = false;
+      if (j < ns) {
+        const uint32_t h = hb[j];  // this thread's own
+        c[u] = ix.slots ? __ldg(reinterpret_cast<const uint32_t*>(ix.slots + (size_t)h * kSlotVecs))
+                        : __ldg(ix.dir + h + 1) - __ldg(ix.dir + h);
+        found[u] = h == ix.empty_hash;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const uint32_t j = j0 + u * G + tid;
+      if (j0 + u * G >= ns) break;  // group-uniform
+      const uint32_t fb = __ballot_sync(FULL, found[u] || c[u] > 0);
+      more |= c[u] > t0;
+      const uint32_t cnt = min(c[u], kE + 1);
+      sq2 += cnt * cnt;
+      if (j < ns) st[j] = (uint16_t)cnt;
+      if (lane == 0 && (j >> 5) < kNW) fm[j >> 5] = fb;
+    }
+  }
+  lg_sync(bar, G);
+  uint32_t ne = 0;
+  {
+    const uint32_t C = (ns + G - 1) / G, lo = min(tid * C, ns), hi = min(lo + C, ns);  // consecutive seeds
+    uint32_t own = 0;
+#pragma unroll 1
+    for (uint32_t j = lo; j < hi; j++) own += st[j];  // at most 2 NS (kE + 1) over all seeds: fits 32 bits
+    uint32_t x = own;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    for (int o = 16; o; o >>= 1) sq2 += min(__shfl_xor_sync(FULL, sq2, o), kLgWork);  // far below 2^32
+    more = __any_sync(FULL, more);
+    if (lane == 31) {
+      red[0][warp] = x;
+      red[1][warp] = min(sq2, kLgWork + 1) | (more ? 0x80000000u : 0u);
+    }
+    if (warp == kW - 1) {  // found seeds before each word: at most 64 words, two a lane
+      const uint32_t nw = (ns + 31) >> 5;
+      const uint32_t c0 = 2 * lane < nw ? __popc(fm[2 * lane]) : 0u,
+                     c1 = 2 * lane + 1 < nw ? __popc(fm[2 * lane + 1]) : 0u;
+      uint32_t f = c0 + c1;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, f, o);
+        if (lane >= (uint32_t)o) f += y;
+      }
+      if (2 * lane < nw) fp[2 * lane] = (uint16_t)(f - c0 - c1);
+      if (2 * lane + 1 < nw) fp[2 * lane + 1] = (uint16_t)(f - c1);
+    }
+    lg_sync(bar, G);
+    uint32_t at = x - own, work = 0, any = 0;
+#pragma unroll 1
+    for (uint32_t w = 0; w < kW; w++) {
+      at += w < warp ? red[0][w] : 0u;
+      ne += red[0][w];
+      work += red[1][w] & 0x7FFFFFFFu;
+      any |= red[1][w];
+    }
+    if (ne > kE || work > kLgWork) return kStrandOverflow;  // group-uniform
+    if (ne == 0) return kStrandOk;  // nothing found: the reference skips the strand
+#pragma unroll 1
+    for (uint32_t j = lo; j < hi; j++) {
+      const uint32_t c = st[j];
+      st[j] = (uint16_t)at;
+      at += c;
+    }
+    if (tid == 0) st[ns] = (uint16_t)ne;
+    more = any >> 31;
+  }
+  lg_sync(bar, G);
+  if (ix.slots)
+#pragma unroll 1
+    for (uint32_t j = tid; j < ns; j += G) {
+      const uint32_t e = st[j], cnt = st[j + 1] - e;
+      if (!cnt) continue;
+      const uint4* sl = ix.slots + (size_t)hb[j] * kSlotVecs;
+      const uint4 v0 = __ldg(sl), v1 = __ldg(sl + 1);
+      uint4 v2 = make_uint4(0u, 0u, 0u, 0u), v3 = v2;
+      if (cnt > 3) {
+        v2 = __ldg(sl + 2);
+        v3 = __ldg(sl + 3);
+      }
       auto put = [&](uint32_t t, uint32_t ref, uint32_t pos) {
         if (t < cnt) {
-          S.p_ref[e + t] = ref;
-          S.p_pos[e + t] = pos;
-          S.p_fj[e + t] = fj;
+          rs[e + t] = (ref << 11) | j;
+          ps[e + t] = pos;
         }
       };
       put(0, v0.z, v0.w);
@@ -177,370 +422,599 @@ __device__ int long_strand(const DevIndex& ix, const uint8_t* raw, uint32_t L, i
       put(4, v2.z, v2.w);
       put(5, v3.x, v3.y);
       put(6, v3.z, v3.w);
-      t0 = kSlotPosts;
     }
-    // the postings past the slot's (all of them without slots), a warp per seed with its lanes on
-    // consecutive postings: each seed's (offset, count, start, fj) goes to the hash set's space,
-    // unused until step 2 (the barriers of the next group's sums order its reuse)
-    uint32_t* o0S = S.hs;
-    uint32_t* cntS = S.hs + G;
-    uint32_t* eS = S.hs + 2 * G;
-    uint32_t* fjS = S.hs + 3 * G;
-    o0S[tid] = o0;
-    cntS[tid] = cnt;
-    eS[tid] = e;
-    fjS[tid] = fj;
-    __syncthreads();
-    {
-      const uint32_t gn = min((uint32_t)G, ns - j0), lane = (uint32_t)tid & 31u;
-      for (uint32_t sd = (uint32_t)tid >> 5; sd < gn; sd += G / 32) {
-        const uint32_t c = cntS[sd];
-        if (c <= t0) continue;  // warp-uniform
-        const uint32_t o = o0S[sd], es = eS[sd], f = fjS[sd];
-        for (uint32_t t = t0 + lane; t < c; t += 32) {
-          const uint2 p = __ldg(ix.post + o + t);
-          S.p_ref[es + t] = p.x;
-          S.p_pos[es + t] = p.y;
-          S.p_fj[es + t] = f;
+  if (more) {  // group-uniform: those past the slots, spread over the threads by posting
+#pragma unroll 1
+    for (uint32_t p0 = tid; p0 < ne; p0 += 4 * G) {
+      uint32_t sj[4];
+      uint2 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {  // up to four loads in flight
+        const uint32_t p = p0 + u * G;
+        sj[u] = kLgEmpty;
+        if (p < ne) {
+          uint32_t lo = 0, hi = ns - 1;  // the last seed that starts at or before p
+#pragma unroll 1
+          while (lo < hi) {
+            const uint32_t mid = (lo + hi + 1) >> 1;
+            if (st[mid] <= p) lo = mid;
+            else hi = mid - 1;
+          }
+          const uint32_t t = p - st[lo];
+          if (t >= t0) {
+            sj[u] = lo;
+            const uint32_t h = hb[lo];
+            const uint32_t o0 =
+                ix.slots ? __ldg(reinterpret_cast<const uint32_t*>(ix.slots + (size_t)h * kSlotVecs) + 1) : __ldg(ix.dir + h);
+            v[u] = __ldg(ix.post + o0 + t);
+          }
         }
       }
-    }
-    nf += fr;
-    ne += er;
-  }
-  __syncthreads();  // the postings in place before step 2 clears the hash set
-  if (ne == 0) return kStrandOk;  // nothing found: the reference skips the strand
-  // 2. occurrence filter: the (refID, found index) set
-  uint32_t hsz = 64;
-  while (hsz < 2 * ne) hsz <<= 1;
-  const uint32_t mask = hsz - 1;
-  for (uint32_t i = tid; i < hsz; i += G) S.hs[i] = kLgEmpty;
-  for (uint32_t i = tid; i < (uint32_t)kLgRT; i += G) S.rt[i] = kLgEmpty;
-  if (tid == 0) {
-    S.n_kept = 0;
-    S.n_rt = 0;
-  }
-  __syncthreads();
-  for (uint32_t i = tid; i < ne; i += G)
-    if (lg_insert(S.hs, mask, (S.p_ref[i] << 11) | (S.p_fj[i] & 0x7FFu), err)) S.p_fj[i] |= 0x80000000u;
-  __syncthreads();
-  // occurrence runs from their first found index: the longest is hs
-  auto run_from = [&](uint32_t i) -> uint32_t {  // 0 unless posting i starts a run
-    const uint32_t fj = S.p_fj[i];
-    if (!(fj >> 31)) return 0;
-    const uint32_t key = (S.p_ref[i] << 11) | (fj & 0x7FFu);
-    if ((fj & 0x7FFu) && lg_contains(S.hs, mask, key - 1, err)) return 0;
-    uint32_t len = 1;
-    while ((fj & 0x7FFu) + len < nf && lg_contains(S.hs, mask, key + len, err)) len++;
-    return len;
-  };
-  uint32_t mx = 0;
-  for (uint32_t i = tid; i < ne; i += G) mx = max(mx, run_from(i));
-  const uint32_t hs = (uint32_t)grp_max_u64<G>(mx, red);
-  // hs only grows on a continued occurrence (Analyser.cpp:2087-2099): below 2 no reference can
-  // reach a diagonal run of 2 either, so the strand has no candidate
-  if (hs < 2) return kStrandOk;
-  const uint32_t keep_min = hs - 1;  // max(1, hs - 1), Analyser.cpp:2115
-  // each insertion attempt first claims a count (n_rt, an upper bound of the distinct references:
-  // threads racing on one reference each claim one): at most kLgRT / 2 insertions happen, so the
-  // table never fills, and a refused one leaves n_rt above kLgRT / 2, which sends the strand to the
-  // block tier
-  for (uint32_t i = tid; i < ne; i += G)
-    if (run_from(i) >= keep_min && !lg_contains(S.rt, kLgRT - 1, S.p_ref[i], err))
-      if (atomicAdd(&S.n_rt, 1u) < (uint32_t)kLgRT / 2) lg_insert(S.rt, kLgRT - 1, S.p_ref[i], err);
-  __syncthreads();
-  if (S.n_rt > (uint32_t)kLgRT / 2) {
-    if (keep_min != 1) return kStrandOverflow;
-    // hs = 2 keeps every reference with a posting (max(1, hs - 1) = 1), more than the table
-    // holds. A diagonal run of 2 needs two postings of one reference on one diagonal at
-    // consecutive seeds ((ref, pos, q) then (ref, pos + step, q + step), Analyser.cpp:2337-2402):
-    // when the strand has no such pair its longest run M is below 2 and it has no candidate. The
-    // pairs are looked for through the hash set, now free, of the postings' (ref, diagonal, seed)
-    // keys folded to 32 bits; a collision can only report a pair that is not there, which sends
-    // the strand on as before.
-    auto dkey = [&](uint32_t i, uint32_t dj) -> uint32_t {
-      const uint32_t j = (S.p_fj[i] >> 11) & 0x7FFu;
-      const uint32_t d = S.p_pos[i] - j * step;  // the diagonal, modulo 2^32
-      const uint64_t x = (uint64_t)S.p_ref[i] * 0x9E3779B97F4A7C15ull ^ (uint64_t)d * 0xC2B2AE3D27D4EB4Full ^
-                         (uint64_t)(j + dj) * 0x165667B19E3779F9ull;
-      const uint32_t v = (uint32_t)(x >> 32) ^ (uint32_t)x;
-      return v == kLgEmpty ? kLgEmpty - 1u : v;
-    };
-    for (uint32_t i = tid; i < hsz; i += G) S.hs[i] = kLgEmpty;
-    __syncthreads();
-    for (uint32_t i = tid; i < ne; i += G) lg_insert(S.hs, mask, dkey(i, 0), err);
-    __syncthreads();
-    int pair = 0;
-    for (uint32_t i = tid; i < ne && !pair; i += G) pair = lg_contains(S.hs, mask, dkey(i, 1), err) ? 1 : 0;
-    if (__syncthreads_or(pair)) return kStrandOverflow;
-    return kStrandOk;  // no diagonal run of 2: no candidate on this strand
-  }
-  // 3. the kept references' postings as (refID << 32 | position, query position) sort keys,
-  //    grouped by reference: the kept references (at most kLgRT / 2) ranked by refID, each one's
-  //    postings counted and given a range in that order, then scattered into it
-  uint64_t* kA = reinterpret_cast<uint64_t*>(S.hs);
-  constexpr int kK = SM::kK;
-  constexpr int kBk = kLgRT / 2;  // ranges
-  uint32_t* kB = S.hs + 2 * kK;
-  if (tid < kLgRT) {
-    const uint32_t r = S.rt[tid];
-    uint32_t rk = 0;
-    if (r != kLgEmpty)
-      for (int s2 = 0; s2 < kLgRT; s2++) {
-        const uint32_t r2 = S.rt[s2];
-        rk += (r2 != kLgEmpty && r2 < r) ? 1u : 0u;
-      }
-    S.rrank[tid] = rk;
-  }
-  if (tid < kBk) {
-    S.bcnt[tid] = 0;
-    S.bfill[tid] = 0;
-  }
-  __syncthreads();
-  for (uint32_t i = tid; i < ne; i += G) {
-    const int sl = lg_find(S.rt, kLgRT - 1, S.p_ref[i], err);
-    if (sl >= 0) atomicAdd(&S.bcnt[S.rrank[sl]], 1u);
-  }
-  __syncthreads();
-  if (tid < 32) {  // the ranges' starts (two per lane), their total and the largest range
-    const unsigned FULL = 0xFFFFFFFFu;
-    const uint32_t c0 = S.bcnt[2 * tid], c1 = S.bcnt[2 * tid + 1];
-    uint32_t x = c0 + c1;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(FULL, x, o);
-      if (tid >= o) x += y;
-    }
-    const uint32_t ex = x - (c0 + c1);
-    S.boff[2 * tid] = ex;
-    S.boff[2 * tid + 1] = ex + c0;
-    if (tid == 31) {
-      S.boff[kBk] = x;
-      S.n_kept = x;
-    }
-    const uint32_t mb = __reduce_max_sync(FULL, max(c0, c1));
-    if (tid == 0) S.bmax = mb;
-  }
-  __syncthreads();
-  const int T2 = (int)S.n_kept;
-  if (T2 > kK) return kStrandOverflow;
-  for (uint32_t i = tid; i < ne; i += G) {
-    const int sl = lg_find(S.rt, kLgRT - 1, S.p_ref[i], err);
-    if (sl >= 0) {
-      const uint32_t b = S.rrank[sl];
-      const uint32_t t = S.boff[b] + atomicAdd(&S.bfill[b], 1u);
-      kA[t] = ((uint64_t)S.p_ref[i] << 32) | S.p_pos[i];
-      kB[t] = ((S.p_fj[i] >> 11) & 0x7FFu) * step;
-    }
-  }
-  __syncthreads();
-  if (S.bmax <= 128u) {
-    // each range sorted by (position, query position), a warp per range: an entry's place is the
-    // number of its range's entries with a smaller key (the keys are distinct), written to the
-    // postings' arrays, free by now, and copied back
-    const uint32_t lane = (uint32_t)tid & 31u, warp = (uint32_t)tid >> 5;
-    for (uint32_t b = warp; b < (uint32_t)kBk; b += G / 32) {
-      const uint32_t b0 = S.boff[b], b1 = S.boff[b + 1];
-      for (uint32_t e = b0 + lane; e < b1; e += 32) {
-        const uint64_t ka = kA[e];
-        const uint32_t kb = kB[e];
-        uint32_t rk = 0;
-        for (uint32_t f = b0; f < b1; f++) {
-          const uint64_t fa = kA[f];
-          rk += (fa < ka || (fa == ka && kB[f] < kb)) ? 1u : 0u;
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (sj[u] != kLgEmpty) {
+          rs[p0 + u * G] = (v[u].x << 11) | sj[u];
+          ps[p0 + u * G] = v[u].y;
         }
-        S.p_ref[b0 + rk] = (uint32_t)(ka >> 32);
-        S.p_pos[b0 + rk] = (uint32_t)ka;
-        S.p_fj[b0 + rk] = kb;
-      }
-    }
-    __syncthreads();
-    for (int i = tid; i < T2; i += G) {
-      kA[i] = ((uint64_t)S.p_ref[i] << 32) | S.p_pos[i];
-      kB[i] = S.p_fj[i];
-    }
-    __syncthreads();
-  } else {  // a large range (a read from one reference): one bitonic sort of all the keys
-    const int N = next_pow2(T2);
-    for (int i = T2 + tid; i < N; i += G) {
-      kA[i] = ~0ull;
-      kB[i] = ~0u;
-    }
-    __syncthreads();
-    bitonic_sort<G>(kA, kB, N);
-  }
-  // 4. diagonal runs (Analyser.cpp:2337-2490): X = position within the run, Y = longest run of
-  //    the reference
-  uint32_t* X = S.p_ref;
-  uint32_t* Y = S.p_pos;
-  auto refA = [&](int i) { return (uint32_t)(kA[i] >> 32); };
-  auto rpos = [&](int i) { return (uint32_t)(kA[i] & 0xFFFFFFFFu); };
-  auto dbrk = [&](int i) {
-    return i == 0 || refA(i) != refA(i - 1) ||
-           !((uint64_t)rpos(i - 1) + step == rpos(i) && (uint64_t)kB[i - 1] + step == kB[i]);
-  };
-  auto rhead = [&](int i) { return i == 0 || refA(i) != refA(i - 1); };
-  auto rtail = [&](int i) { return i == T2 - 1 || refA(i) != refA(i + 1); };
-  arr_seg_scan<G, false>(X, T2, [&](int) -> uint32_t { return 1u; }, dbrk, OpAdd(), red);
-  arr_seg_scan<G, false>(Y, T2, [&](int i) -> uint32_t { return X[i]; }, rhead, OpMax(), red);
-  arr_seg_scan<G, true>(Y, T2, [&](int i) -> uint32_t { return Y[i]; }, rtail, OpMax(), red);
-  uint32_t mr = 0;
-  {
-    const int C = (T2 + G - 1) / G;
-    for (int i = tid * C; i < T2 && i < (tid + 1) * C; i++) mr = Y[i] > mr ? Y[i] : mr;
-  }
-  const uint32_t M = (uint32_t)grp_max_u64<G>(mr, red);
-  if (M < 2) return kStrandOk;  // Analyser.cpp:2402
-  // 5. head/tail walks of every run of a reference whose longest run is M: the run's covered
-  //    interval [Start.Q - head, Start.Q - head + T) and T go to X at the run's last entry
-  {
-    const int C = (T2 + G - 1) / G;
-    for (int i = tid * C; i < T2 && i < (tid + 1) * C; i++) {
-      uint32_t z = 0;
-      const bool rend = (i == T2 - 1) || dbrk(i + 1);
-      if (rend && Y[i] == M) {
-        const int s = i - (int)X[i] + 1;
-        const uint32_t ref = refA(i);
-        const uint32_t sr = rpos(s), sq = kB[s];
-        const uint32_t lr = rpos(i) + step, lq = kB[i] + step;
-        const uint8_t* rs = ix.bases + ix.ref_off[ref];
-        const uint32_t rlen = ix.ref_len[ref];
-        const uint32_t tail = tail_walk(S.q, rs, L, rlen, lq, lr, k);
-        const uint32_t head = head_walk(S.q, rs, sq, sr, k);
-        const uint32_t tot = tail + head + (lq - sq);
-        if (tot >= k) z = ((sq - head) << 16) | tot;
-      }
-      X[i] = z;
     }
   }
-  __syncthreads();
-  // 6. candidates in ascending refID: the heads of the reference segments whose longest run is M
-  uint32_t n_cand;
-  {
-    const int C = (T2 + G - 1) / G;
-    uint32_t local = 0;
-    for (int i = tid * C; i < T2 && i < (tid + 1) * C; i++) local += (rhead(i) && Y[i] == M);
-    uint32_t at = grp_excl_sum<G>(local, red, &n_cand);
-    __syncthreads();
-    for (int i = tid * C; i < T2 && i < (tid + 1) * C; i++)
-      if (rhead(i) && Y[i] == M) kB[at++] = (uint32_t)i;  // kB's query positions are walked by now
-  }
-  __syncthreads();
-  // 7. scores, a warp per candidate (Analyser.cpp:2490-2540, MatrixCPU.cpp:18-214): the candidate's
-  //    reference segment [sa, sb) of the sorted keys, its walked runs' lengths summed (sc) and summed
-  //    as triangles (sr), the query bases they cover counted in the warp's own bitmap; a candidate
-  //    whose runs all fell short of k keeps Score -2 and is not scored. Then the scored ones in
-  //    ascending refID, and the highest relative score in that order.
-  if (n_cand > (uint32_t)kLgC) return kStrandOverflow;  // group-uniform (n_rt bounds it first)
-  const uint32_t nw = (L + 31) / 32;
-  const uint32_t lane = (uint32_t)tid & 31u, warp = (uint32_t)tid >> 5;
-  const uint32_t n_warps = min((uint32_t)(G / 32), (uint32_t)SM::kE / nw);  // bitmaps fit p_fj
-  if (tid < kLgC / 32) S.scored[tid] = 0;
-  __syncthreads();
-  mg_candidate* out = S.cb[strand];
-  if (warp < n_warps) {
-    uint32_t* cov = S.p_fj + warp * nw;
-    for (uint32_t c = warp; c < n_cand; c += n_warps) {
-      const int sa = (int)kB[c];
-      const uint32_t ref = refA(sa);
-      uint32_t first = (uint32_t)T2;
-      for (int i = sa + 1 + (int)lane; i < T2; i += 32)
-        if (refA(i) != ref) {
-          first = (uint32_t)i;
-          break;
-        }
-      const int sb = (int)__reduce_min_sync(0xFFFFFFFFu, first);
-      uint32_t sc = 0;
-      uint64_t sr = 0;
-      for (int i = sa + (int)lane; i < sb; i += 32) {
-        const uint32_t z = X[i];
-        if (z) {
-          const uint64_t t = z & 0xFFFFu;
-          sc += (uint32_t)t;
-          sr += (t * (t + 1)) / 2;
-        }
-      }
-      sc = __reduce_add_sync(0xFFFFFFFFu, sc);  // at most kK runs of < 2^16 bases each
-      for (int o = 16; o; o >>= 1) sr += __shfl_xor_sync(0xFFFFFFFFu, sr, o);
-      if (sc == 0) continue;  // warp-uniform: Score stays -2
-      for (uint32_t w = lane; w < nw; w += 32) cov[w] = 0;
-      __syncwarp();
-      for (int i = sa + (int)lane; i < sb; i += 32) {
-        const uint32_t z = X[i];
-        if (!z) continue;
-        const uint32_t a = z >> 16, bnd = a + (z & 0xFFFFu);
-        for (uint32_t wd = a >> 5; wd <= (bnd - 1) >> 5; wd++) {
-          const uint32_t w0 = wd * 32;
-          const uint32_t lo = a > w0 ? a : w0, up = bnd < w0 + 32 ? bnd : w0 + 32;
-          const uint32_t n = up - lo;
-          atomicOr(&cov[wd], (n == 32 ? 0xFFFFFFFFu : ((1u << n) - 1u)) << (lo - w0));
-        }
-      }
-      __syncwarp();
-      uint32_t hits = 0;
-      for (uint32_t w = lane; w < nw; w += 32) hits += __popc(cov[w]);
-      hits = __reduce_add_sync(0xFFFFFFFFu, hits);
-      if (lane == 0) {
-        float score, pct;
-        final_score(sr, (uint64_t)sc, hits, L, &score, &pct);
-        const float rel = relative_score(ix, __uint2float_rn(L), __uint2float_rn(ix.ref_len[ref]), score, err);
-        out[c] = mg_candidate{ref, rel, score, pct};
-        atomicOr(&S.scored[c >> 5], 1u << (c & 31u));
-      }
-      __syncwarp();  // the bitmap's next clear after this candidate's count
+  lg_sync(bar, G);
+  const uint32_t fw = (ns - 1) >> 5;
+  const uint32_t nf = fp[fw] + __popc(fm[fw]), nfw = (nf + 31) >> 5;
+  // 2. the linked references (the warps reconverge between the two searches)
+#pragma unroll 1
+  for (uint32_t i0 = 0; i0 < ne; i0 += G) {
+    const uint32_t i = i0 + tid, x = i < ne ? rs[i] : 0u, j = x & 2047u;
+    uint32_t w = j >> 5, m = i < ne ? fm[w] & ((1u << (j & 31u)) - 1u) : 0u;
+#pragma unroll 1
+    while (!m && w && i < ne) m = fm[--w];
+    uint32_t a = 0, c = 0, t = 0;
+    if (m) {
+      const uint32_t pj = w * 32 + 31 - __clz(m);
+      a = st[pj];
+      c = st[pj + 1] - a;
+      t = i - st[j];  // a stray hit in either bucket shifts the copies by one
+      t = t < 2 ? 0 : t - 2;
+      if (t >= c) t = 0;
     }
-  }
-  __syncthreads();
-  if (warp == 0) {  // in place: a scored candidate only moves down, after its chunk is read
-    uint32_t n_sc = 0;
-    for (uint32_t c0 = 0; c0 < n_cand; c0 += 32) {
-      const uint32_t c = c0 + lane;
-      const bool ok = c < n_cand && ((S.scored[c >> 5] >> (c & 31u)) & 1u);
-      mg_candidate v{};
-      if (ok) v = out[c];
-      const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
-      __syncwarp();
-      if (ok) out[n_sc + __popc(m & ((1u << lane) - 1u))] = v;
-      n_sc += __popc(m);
+    bool linked = false;
+#pragma unroll 1
+    for (uint32_t n = 0; n < c && !linked; n++) {
+      linked = (rs[a + t] ^ x) < 2048u;
+      if (++t == c) t = 0;
     }
     __syncwarp();
-    if (lane == 0) {
-      float hi = -1.0f;
-      for (uint32_t i = 0; i < n_sc; i++)
-        if (out[i].rel > hi) hi = out[i].rel;
-      S.n_sc = n_sc;
-      S.hi = hi;
+    const uint32_t ref = x >> 11;
+    uint32_t s = lg_mix(ref) & (kRT - 1), left = linked ? kRT : 0u;  // each slot once
+#pragma unroll 1
+    while (left) {
+      uint32_t old = *(volatile uint32_t*)&T.rt[s];
+      if (old == kLgEmpty && !*(volatile uint32_t*)&S.over[half]) {  // the table stays free to end probes
+        old = atomicCAS(&T.rt[s], kLgEmpty, ref);
+        if (old == kLgEmpty) {
+          const uint32_t id = atomicAdd(&S.n_rt[half], 1u);
+          if (id < kRM) {
+            T.rid[s] = (uint8_t)id;
+            iref[id] = ref;
+          } else {
+            S.over[half] = 1;
+          }
+        }
+      }
+      left = old == ref || old == kLgEmpty ? 0u : left - 1;
+      s = (s + 1) & (kRT - 1);
+    }
+    __syncwarp();
+  }
+  lg_sync(bar, G);
+  const uint32_t R = S.n_rt[half];
+  if (R == 0) return kStrandOk;  // no reference at two found seeds in a row: no candidate
+  // the bitmaps (R of nfw words) and, behind them, the ones before each word (R nfw half-words) lie over sx
+  if (R > kRM || 3 * R * nfw > kE / 2) return kStrandOverflow;
+  // 3. occurrence filter; from here on the postings hold, in place of the refID, its reference's order
+  //    of insertion (kNoId: not linked, not needed any more)
+  constexpr uint32_t kNoId = 127;
+  uint32_t* bm = reinterpret_cast<uint32_t*>(sx);
+  uint16_t* pw = sx + 2 * R * nfw;
+#pragma unroll 1
+  for (uint32_t i = tid; i < R * nfw; i += G) bm[i] = 0;
+  if (tid == 0) S.dup[half] = 0;
+  lg_sync(bar, G);
+  const uint32_t only = iref[0];
+#pragma unroll 1
+  for (uint32_t i0 = 0; i0 < ne; i0 += G) {
+    const uint32_t i = i0 + tid, x = i < ne ? rs[i] : kLgEmpty, ref = x >> 11, j = x & 2047u;
+    uint32_t id = kNoId;
+    if (R == 1) {
+      if (i < ne && ref == only) id = 0;
+    } else {
+      uint32_t s = lg_mix(ref) & (kRT - 1), left = i < ne ? kRT : 0u;  // the table has free slots: R <= kRM < kRT
+#pragma unroll 1
+      while (left) {
+        const uint32_t v = T.rt[s];
+        if (v == ref) id = T.rid[s];
+        left = v == ref || v == kLgEmpty ? 0u : left - 1;
+        s = (s + 1) & (kRT - 1);
+      }
+    }
+    __syncwarp();
+    if (i < ne) {
+      rs[i] = (id << 11) | j;
+      if (id != kNoId) {
+        const uint32_t f = fp[j >> 5] + __popc(fm[j >> 5] & ((1u << (j & 31u)) - 1u)), bit = 1u << (f & 31u);
+        if (atomicOr(&bm[id * nfw + (f >> 5)], bit) & bit) S.dup[half] = 1;  // twice under one seed
+      }
     }
   }
-  __syncthreads();
-  const uint32_t n_sc = S.n_sc;
-  const float hi = S.hi;
-  __syncthreads();  // S.n_sc and S.hi read before the next strand writes them
-  *n_out = n_sc;
-  *highest = hi;
+  lg_sync(bar, G);
+  if (nfw == 1) {
+#pragma unroll 1
+    for (uint32_t id = tid; id < R; id += G) {
+      best[id] = (uint16_t)longest_run(bm[id]);
+      T.cnt[id] = (uint16_t)__popc(bm[id]);
+      pw[id] = 0;
+    }
+  } else {
+#pragma unroll 1
+    for (uint32_t id = warp; id < R; id += kW) {
+      uint32_t n;
+      const uint32_t b = warp_longest_run(bm + id * nfw, nfw, pw + id * nfw, &n);
+      if (lane == 0) {
+        best[id] = (uint16_t)b;
+        T.cnt[id] = (uint16_t)n;
+      }
+    }
+  }
+  lg_sync(bar, G);
+  uint32_t hs = 0;
+#pragma unroll 1
+  for (uint32_t id = lane; id < R; id += 32) hs = max(hs, (uint32_t)best[id]);
+  hs = __reduce_max_sync(FULL, hs);
+  const uint32_t keep_min = max(2u, hs - 1);  // max(1, hs - 1) (Analyser.cpp:2115), among the linked
+  uint32_t nk = 0;  // kept references
+#pragma unroll 1
+  for (uint32_t i0 = 0; i0 < R; i0 += 32) nk += __popc(__ballot_sync(FULL, i0 + lane < R && best[i0 + lane] >= keep_min));
+#pragma unroll 1
+  for (uint32_t id = tid; id < R; id += G) {
+    uint32_t r = kNoId;
+    if (best[id] >= keep_min) {
+      const uint32_t ref = iref[id];
+      r = 0;
+#pragma unroll 4
+      for (uint32_t u = 0; u < R; u++) r += (best[u] >= keep_min && iref[u] < ref) ? 1u : 0u;
+      T.kref[r] = ref;
+      T.kid[r] = (uint8_t)id;
+    }
+    T.rk[id] = (uint8_t)r;
+  }
+#pragma unroll 1
+  for (uint32_t i = tid; i < kRM; i += G) T.segmax[i] = 0;
+  lg_sync(bar, G);
+  auto rank_of = [&](uint32_t x) -> uint32_t { return T.rk[(x >> 11) & 127u]; };  // of a linked posting
+  // 4. the kept postings in (refID, position, seed) order, as indices in sx[0 .. T2)
+  auto key_of = [&](uint32_t i) { return ((uint64_t)ps[i] << 11) | (rs[i] & 2047u); };
+  uint32_t T2 = 0;
+  // a range [a, b) of kept postings ranked by a warp into dst: an entry's place is the number of
+  // smaller keys (the keys are distinct)
+  auto rank_range = [&](const uint16_t* src, uint16_t* dst, uint32_t a, uint32_t b) {
+#pragma unroll 1
+    for (uint32_t e0 = a; e0 < b; e0 += 32) {
+      const uint32_t e = e0 + lane;
+      const uint32_t mine = e < b ? src[e] : 0u;
+      const uint64_t key = e < b ? key_of(mine) : 0ull;
+      uint32_t r = 0;
+#pragma unroll 1
+      for (uint32_t f0 = a; f0 < b; f0 += 32) {
+        const uint64_t other = f0 + lane < b ? key_of(src[f0 + lane]) : ~0ull;
+        const uint32_t n = min(32u, b - f0);
+#pragma unroll 4
+        for (uint32_t u = 0; u < n; u++) r += __shfl_sync(FULL, other, u) < key ? 1u : 0u;
+      }
+      if (e < b) dst[a + r] = (uint16_t)mine;
+    }
+  };
+  const bool dup = S.dup[half] != 0;
+  uint32_t* badr = bk;  // ranges with postings out of order, a bit each
+  if (dup) {  // a reference twice under a seed: the postings are counted one by one
+#pragma unroll 1
+    for (uint32_t id = tid; id < R; id += G) bfill[id] = 0;
+    lg_sync(bar, G);
+#pragma unroll 1
+    for (uint32_t i = tid; i < ne; i += G) {  // a posting's place in its range goes beside its id
+      const uint32_t x = rs[i];
+      if ((x >> 11) != kNoId && rank_of(x) != kNoId) rs[i] = x | (atomicAdd(&bfill[x >> 11], 1u) << 18);
+    }
+    lg_sync(bar, G);
+#pragma unroll 1
+    for (uint32_t id = tid; id < R; id += G) T.cnt[id] = (uint16_t)bfill[id];
+    lg_sync(bar, G);
+  }
+  uint32_t bmax = 0;
+#pragma unroll 1
+  for (uint32_t b0 = 0; b0 < nk; b0 += 32) {  // every warp: the ranges' starts; warp 0 writes them
+    const uint32_t b = b0 + lane, c = b < nk ? T.cnt[T.kid[b]] : 0u;
+    uint32_t x = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    if (warp == 0 && b < nk) boff[b] = (uint16_t)(T2 + x - c);
+    T2 += __shfl_sync(FULL, x, 31);
+    bmax = max(bmax, __reduce_max_sync(FULL, c));
+  }
+  if (T2 > kE / 2) return kStrandOverflow;  // group-uniform
+  if (tid == 0) boff[nk] = (uint16_t)T2;
+  if (tid < (kRM + 31) / 32) badr[tid] = 0;
+  lg_sync(bar, G);
+#pragma unroll 1
+  for (uint32_t i = tid; i < ne; i += G) {  // into the ranges, in seed order unless dup
+    const uint32_t x = rs[i], id = (x >> 11) & 127u;
+    if (id == kNoId) continue;
+    const uint32_t b = T.rk[id];
+    if (b == kNoId) continue;
+    uint32_t at = x >> 18;
+    if (!dup) {
+      const uint32_t j = x & 2047u, f = fp[j >> 5] + __popc(fm[j >> 5] & ((1u << (j & 31u)) - 1u));
+      const uint32_t w = id * nfw + (f >> 5);
+      at = pw[w] + __popc(bm[w] & ((1u << (f & 31u)) - 1u));
+    }
+    kl[boff[b] + at] = (uint16_t)i;
+  }
+  lg_sync(bar, G);
+  bool bad = dup;  // seed order is not position order: a stray hit, or copies within the reference
+#pragma unroll 1
+  for (uint32_t i = tid; i < T2; i += G) {
+    const uint32_t a = kl[i];
+    if (i > 0) {
+      const uint32_t p = kl[i - 1];
+      const uint32_t b = rank_of(rs[a]);
+      if (rank_of(rs[p]) == b && key_of(p) > key_of(a)) {
+        bad = true;
+        atomicOr(&badr[b >> 5], 1u << (b & 31u));
+      }
+    }
+    sx[i] = (uint16_t)a;
+  }
+  bad = __any_sync(FULL, bad);
+  if (lane == 0) red[1][warp] = bad;
+  lg_sync(bar, G);
+  uint32_t any = 0;
+#pragma unroll 1
+  for (uint32_t w = 0; w < kW; w++) any |= red[1][w];
+  bool sorted = !any;
+  if (!sorted && bmax <= kRankMax) {
+#pragma unroll 1
+    for (uint32_t b = warp; b < nk; b += kW)
+      if (dup || ((badr[b >> 5] >> (b & 31u)) & 1u)) rank_range(kl, sx, boff[b], boff[b + 1]);
+    sorted = true;
+    lg_sync(bar, G);
+  }
+  if (!sorted) {  // a reference with many postings out of order: bitonic sort of the indices
+    uint32_t N = 2;
+#pragma unroll 1
+    while (N < T2) N <<= 1;
+#pragma unroll 1
+    for (uint32_t i = T2 + tid; i < N; i += G) sx[i] = 0xFFFFu;
+    lg_sync(bar, G);
+#pragma unroll 1
+    for (uint32_t kk = 2; kk <= N; kk <<= 1) {
+#pragma unroll 1
+      for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
+#pragma unroll 1
+        for (uint32_t c = tid; c < N / 2; c += G) {
+          const uint32_t i = 2 * c - (c & (jj - 1)), p = i + jj;  // the pairs i, i ^ jj with i the lower
+          const uint32_t a = sx[i], b = sx[p];
+          bool gt;
+          if (a == 0xFFFFu || b == 0xFFFFu) {
+            gt = a > b;
+          } else {
+            const uint32_t ra = rank_of(rs[a]), rb = rank_of(rs[b]);
+            gt = ra > rb || (ra == rb && key_of(a) > key_of(b));
+          }
+          if (gt == ((i & kk) == 0) && a != b) {
+            sx[i] = (uint16_t)b;
+            sx[p] = (uint16_t)a;
+          }
+        }
+        lg_sync(bar, G);
+      }
+    }
+  }
+  // 5. diagonal runs (Analyser.cpp:2337-2490): run starts, and each reference's longest run
+#pragma unroll 1
+  for (uint32_t i0 = 0; i0 < T2; i0 += G) {
+    const uint32_t i = i0 + tid;
+    bool start = true;
+    if (i < T2 && i > 0) {
+      const uint32_t a = sx[i - 1], b = sx[i];
+      // one reference and seed + 1: one addition on the packed word
+      const uint32_t xa = rs[a] & 0x3FFFFu, xb = rs[b] & 0x3FFFFu;
+      start = !((uint64_t)ps[a] + step == ps[b] && xa + 1u == xb && (xb & 2047u) != 0);
+    }
+    const uint32_t w = __ballot_sync(FULL, start);
+    if (lane == 0 && (i0 + warp * 32) < T2) bk[(i0 >> 5) + warp] = w;
+  }
+  lg_sync(bar, G);
+  auto run_end = [&](uint32_t i) { return i + 1 == T2 || ((bk[(i + 1) >> 5] >> ((i + 1) & 31u)) & 1u); };
+  auto run_first = [&](uint32_t i) {  // bit 0 is set: the search ends there at the latest
+    uint32_t w = i >> 5, m = bk[w] & (0xFFFFFFFFu >> (31u - (i & 31u)));
+#pragma unroll 1
+    while (!m) m = bk[--w];
+    return w * 32 + 31 - __clz(m);
+  };
+  if (tid == 0) S.n_ends[half] = 0;
+#pragma unroll 1
+  for (uint32_t i = tid; i < T2; i += G)
+    if (run_end(i)) atomicMax(&T.segmax[rank_of(rs[sx[i]])], i - run_first(i) + 1);
+  lg_sync(bar, G);
+  uint32_t M = 0;
+#pragma unroll 1
+  for (uint32_t b = lane; b < nk; b += 32) M = max(M, T.segmax[b]);
+  M = __reduce_max_sync(FULL, M);
+  if (M < 2) return kStrandOk;  // Analyser.cpp:2402
+  *wide = hs == 2 && ne > kLgKeepAll;
+  // 6. candidates: the kept references whose longest run is M, in rank order (every warp has the
+  //    masks); the walks of all their runs, a run end a thread, summed per candidate, as many
+  //    candidates at a time as their coverage bitmaps have room
+  constexpr uint32_t kCM = (kRM + 31) / 32;
+  uint32_t cm[kCM];
+  uint32_t nc = 0;
+#pragma unroll
+  for (uint32_t u = 0; u < kCM; u++) {
+    const uint32_t b = u * 32 + lane;
+    cm[u] = __ballot_sync(FULL, b < nk && T.segmax[b] == M);
+    nc += __popc(cm[u]);
+  }
+  auto cand_of = [&](uint32_t b) -> int {  // a rank's candidate, -1: none
+    uint32_t before = 0;
+    int c = -1;
+#pragma unroll
+    for (uint32_t u = 0; u < kCM; u++) {
+      if ((b >> 5) == u && ((cm[u] >> (b & 31u)) & 1u)) c = (int)(before + __popc(cm[u] & ((1u << (b & 31u)) - 1u)));
+      before += __popc(cm[u]);
+    }
+    return c;
+  };
+  const uint32_t nw = (L + 31) / 32;
+  uint32_t* cov = reinterpret_cast<uint32_t*>(st);
+  const uint32_t per = kCovWords / nw;
+#pragma unroll 1
+  for (uint32_t c = tid; c < nc; c += G) {
+    T.sumc[c] = 0;
+    T.sumr[c] = 0;
+  }
+#pragma unroll 1
+  for (uint32_t i0 = 0; i0 < T2; i0 += G) {  // the candidates' run ends, listed (in kl) to fill the warps
+    const uint32_t i = i0 + tid;
+    const bool end = i < T2 && run_end(i) && T.segmax[rank_of(rs[sx[i]])] == M;
+    const uint32_t m = __ballot_sync(FULL, end);
+    if (!m) continue;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&S.n_ends[half], (uint32_t)__popc(m));
+    at = __shfl_sync(FULL, at, 0);
+    if (end) kl[at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)i;
+  }
+  lg_sync(bar, G);  // every warp has its masks: segmax holds the covered bases from here on
+  const uint32_t n_ends = S.n_ends[half];
+#pragma unroll 1
+  for (uint32_t c0 = 0; c0 < nc; c0 += per) {
+    const uint32_t cn = min(per, nc - c0);
+#pragma unroll 1
+    for (uint32_t i = tid; i < cn * nw; i += G) cov[i] = 0;
+    lg_sync(bar, G);
+#pragma unroll 1
+    for (uint32_t t0 = 0; t0 < n_ends; t0 += G) {
+      const uint32_t t = t0 + tid;
+      int c = -1;
+      uint32_t z = 0, i = 0, xe = 0, rank = 0;
+      if (t < n_ends) {
+        i = kl[t];
+        xe = rs[sx[i]];
+        rank = rank_of(xe);
+        c = cand_of(rank);
+      }
+      if (c >= (int)c0 && c < (int)(c0 + cn)) {
+        const uint32_t s = sx[run_first(i)];
+        z = walk_run(ix, S.comp, raw, L, strand, T.kref[rank], ps[s], ps[sx[i]] + step,
+                     (rs[s] & 2047u) * step, (xe & 2047u) * step + step, k);
+      }
+      __syncwarp();
+      if (!z) continue;
+      const uint32_t len = z & 0xFFFFu, a = z >> 16, bnd = a + len;
+      atomicAdd(&T.sumc[c], len);
+      atomicAdd(&T.sumr[c], (unsigned long long)len * (len + 1) / 2);
+      uint32_t* cv = cov + (c - c0) * nw;
+#pragma unroll 1
+      for (uint32_t wd = a >> 5; wd <= (bnd - 1) >> 5; wd++) {
+        const uint32_t w0 = wd * 32;
+        const uint32_t lo = a > w0 ? a : w0, up = bnd < w0 + 32 ? bnd : w0 + 32;
+        const uint32_t n = up - lo;
+        atomicOr(&cv[wd], (n == 32 ? 0xFFFFFFFFu : ((1u << n) - 1u)) << (lo - w0));
+      }
+    }
+    lg_sync(bar, G);
+#pragma unroll 1
+    for (uint32_t c = warp; c < cn; c += kW) {
+      uint32_t hits = 0;
+#pragma unroll 1
+      for (uint32_t w = lane; w < nw; w += 32) hits += __popc(cov[c * nw + w]);
+      hits = __reduce_add_sync(FULL, hits);
+      if (lane == 0) T.segmax[c0 + c] = hits;
+    }
+    lg_sync(bar, G);
+  }
+  // 7. scores, a lane per candidate (MatrixCPU.cpp:18-214); one whose runs all fell short of k keeps
+  //    Score -2 and is not scored
+  if (warp == 0) {
+    uint32_t n_sc = 0;
+    float hi = -1.0f;
+#pragma unroll 1
+    for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
+      const uint32_t c = c0 + lane;
+      const bool ok = c < nc && T.sumc[c] > 0;
+      uint32_t ref = 0;
+      float score = 0.0f, pct = 0.0f, rel = -1.0f;
+      if (ok) {
+        uint32_t n = c;  // the candidate's rank: the c-th set bit of the masks
+        bool have = false;
+#pragma unroll
+        for (uint32_t u = 0; u < kCM; u++) {
+          const uint32_t pc = __popc(cm[u]);
+          if (!have && n < pc) {
+            ref = T.kref[u * 32 + __fns(cm[u], 0, (int)n + 1)];
+            have = true;
+          }
+          if (!have) n -= pc;
+        }
+        final_score(T.sumr[c], (uint64_t)T.sumc[c], T.segmax[c], L, &score, &pct);
+        rel = relative_score_tab(ix, L, ix.ref_len[ref], score, err);
+      }
+      const uint32_t m = __ballot_sync(FULL, ok);
+      if (ok) cb[n_sc + __popc(m & ((1u << lane) - 1u))] = mg_candidate{ref, rel, score, pct};
+      n_sc += __popc(m);
+      hi = fmaxf(hi, rel);
+    }
+    for (int o = 16; o; o >>= 1) hi = fmaxf(hi, __shfl_xor_sync(FULL, hi, o));
+    if (lane == 0) {
+      S.n_out[half] = n_sc;
+      S.hi[half] = hi;
+    }
+  }
+  lg_sync(bar, G);
+  *n_out = S.n_out[half];
+  *highest = S.hi[half];
   return kStrandOk;
 }
 
-// Both strands of read r, the strand merge and the staging write; false when the read must go
-// to the next tier.
+// Whether the read's L bytes are all letters of ACGT in either case (1), or else all have a
+// complement (0), or not (-1); on the whole block.
+template <class SM>
+__device__ int read_letters(const uint8_t* raw, uint32_t L, const SM& S) {
+  const uintptr_t a = (uintptr_t)raw, e = a + L;
+  bool other = false;
+#pragma unroll 1
+  for (uintptr_t w = (a & ~(uintptr_t)3) + 4 * threadIdx.x; L && w < e; w += 4 * blockDim.x) {
+    uint32_t x = *(const uint32_t*)w;  // an aligned word holding at least one byte of the read
+    if (w < a) x = (x & (0xFFFFFFFFu << (8 * (uint32_t)(a - w)))) | (0x41414141u >> (32 - 8 * (uint32_t)(a - w)));
+    if (w + 4 > e) {
+      const uint32_t o = 8 * (uint32_t)(w + 4 - e);
+      x = (x & (0xFFFFFFFFu >> o)) | (0x41414141u << (32 - o));
+    }
+    other |= !acgt4(upper4(x));
+  }
+  if (!__syncthreads_or(other)) return 1;
+  bool bad = false;
+#pragma unroll 1
+  for (uint32_t i = threadIdx.x; i < L; i += blockDim.x) bad |= S.comp[raw[i]] == 0;
+  return __syncthreads_or(bad) ? -1 : 0;
+}
+
+// Both strands of read r, the strand merge and the staging write; false when the read must go to the
+// next tier. n_small, n_large (optional): counters of the reads that the halves, and the block with
+// its table of kept references, could not take. ahead (thread 0's): the entry of list that the block
+// takes next; while the first warp writes this read's result, the last one asks for that read's bases.
 template <class SM>
 __device__ bool process_read_long(const DevIndex& ix, const BatchDev& b, uint32_t r, SM& S, mg_candidate* stage,
-                                  mg_candidate* arena, uint64_t arena_cap, unsigned long long* arena_n, int* errw) {
+                                  mg_candidate* arena, uint64_t arena_cap, unsigned long long* arena_n, int* errw,
+                                  unsigned* n_small, unsigned* n_large, const uint32_t* list = nullptr,
+                                  uint32_t n_list = 0, uint32_t ahead = 0) {
+  constexpr int H = SM::H;
   const uint64_t o0 = b.offs[r];
   const uint64_t Lr = b.offs[r + 1] - o0;
-  if (Lr > (uint64_t)SM::kQ || ix.n_refs > (1u << 21)) return false;  // keys hold refID << 11
+  if (Lr > (uint64_t)kLgQ || ix.n_refs > (1u << 21)) {  // the packed postings hold refID << 11
+    if (threadIdx.x == 0 && n_small) {
+      atomicAdd(n_small, 1u);
+      atomicAdd(n_large, 1u);
+    }
+    return false;
+  }
   const uint32_t L = (uint32_t)Lr;
   const uint8_t* raw = b.bases + o0;
+  const int letters = read_letters(raw, L, S);
+  if (letters < 0) {
+    if (threadIdx.x == 0) {
+      b.reads[r] = mg_read_result{-1.0f, 0, 0, 0, MG_READ_BAD_BYTE, 0, 0};
+      atomicOr(errw, kErrBadInput);
+    }
+    return true;
+  }
   int err = 0;
   uint32_t n[2] = {0, 0};
   float h[2] = {-1.0f, -1.0f};
-  int st = long_strand(ix, raw, L, 0, S, &err, &n[0], &h[0]);
-  if (st != kStrandBad && st != kStrandOverflow) st = long_strand(ix, raw, L, 1, S, &err, &n[1], &h[1]);
-  if (err) atomicOr(errw, err);  // any thread's: the probes and the scoring lanes record bits per thread
-  if (st == kStrandOverflow) return false;
-  if (threadIdx.x == 0)
-    write_read_result_s(b, r, st == kStrandBad, n[0], n[1], h[0], h[1], S.cb[0], S.cb[1], stage, arena, arena_cap,
-                        arena_n, errw, err);
+  bool wide = false, over = false;
+  // first the strands side by side, then, when one does not fit its half, in turn on the whole block
+#pragma unroll 1
+  for (int pass = 0; pass < 3; pass++) {
+    const bool whole = pass > 0;
+    const int half = whole ? 0 : threadIdx.x / H, strand = whole ? pass - 1 : half;
+    uint32_t n1;
+    float h1;
+    bool w = false;
+    const int s = long_strand(ix, raw, L, strand, letters == 1, S, whole, half, S.cb[strand], &err, &n1, &h1, &w);
+    __syncthreads();
+    if (threadIdx.x % H == 0 && (!whole || threadIdx.x == 0)) {
+      S.status[strand] = s;
+      S.n_out[strand] = n1;
+      S.hi[strand] = h1;
+      if (w) S.handed = 1;  // a strand outside the kept-reference tables, finished here
+      if (threadIdx.x == 0) S.ahead = ahead;
+    }
+    __syncthreads();
+    if (!whole) {
+      n[0] = S.n_out[0];
+      n[1] = S.n_out[1];
+      h[0] = S.hi[0];
+      h[1] = S.hi[1];
+      over = S.status[0] != kStrandOk || S.status[1] != kStrandOk;
+    } else {
+      over = S.status[strand] != kStrandOk;
+      (strand ? n[1] : n[0]) = S.n_out[strand];
+      (strand ? h[1] : h[0]) = S.hi[strand];
+    }
+    wide = S.handed != 0;
+    __syncthreads();
+    if (pass == 0 && threadIdx.x == 0 && n_small && (over || wide)) atomicAdd(n_small, 1u);
+    if (over == whole) break;  // both strands done on the halves, or one does not fit at all
+    if (pass == 0 && threadIdx.x == 0) S.handed = 0;
+  }
+  if (threadIdx.x == 0) S.handed = 0;
+  if (threadIdx.x == 0 && n_large && (over || wide)) atomicAdd(n_large, 1u);
+  if (err) atomicOr(errw, err);  // any thread's: the scoring lanes record bits per thread
+  if (over) return false;
+  // the strand merge (Analyser.cpp:592-611), the log skip rule (:388) and the staging write
+  const int ch = h[0] < h[1] ? 1 : 0;  // Analyser.cpp:601
+  const uint32_t tot = n[0] + n[1];
+  if (threadIdx.x < 32) {
+    uint32_t top = 0;
+#pragma unroll 1
+    for (uint32_t c = threadIdx.x; c < n[ch]; c += 32) top += S.cb[ch][c].rel == h[ch];
+    top = __reduce_add_sync(0xffffffffu, top);
+    if (threadIdx.x == 0) {
+      unsigned long long at = 0;
+      bool fits = true;
+      if (tot > (uint32_t)kSlots) {
+        at = atomicAdd(arena_n, (unsigned long long)tot);
+        fits = at + tot <= arena_cap;
+        if (!fits) atomicOr(errw, kErrArena);
+      }
+      S.cand_at = fits ? (uint32_t)at : kLgEmpty;
+      b.reads[r] = mg_read_result{h[ch], fits ? (uint32_t)at : 0u, (uint16_t)n[0], (uint16_t)n[1], (uint8_t)ch,
+                                  (uint8_t)((n[ch] > 0 && h[ch] != 0.0f) ? 1 : 0), (uint16_t)top};
+    }
+  } else if (list && threadIdx.x >= 2 * H - 32 && S.ahead < n_list) {
+    const uint32_t r2 = list[S.ahead];
+    const uint64_t a = b.offs[r2], e = b.offs[r2 + 1];
+    if (e - a <= (uint64_t)kLgQ)
+#pragma unroll 1
+      for (uint64_t o = a + 128 * (threadIdx.x & 31u); o < e; o += 128 * 32)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(b.bases + o));
+  }
   __syncthreads();
+  if (S.cand_at != kLgEmpty) {
+    mg_candidate* dst = tot > (uint32_t)kSlots ? arena + S.cand_at : stage + (uint64_t)r * kSlots;
+#pragma unroll 1
+    for (uint32_t c = threadIdx.x; c < tot; c += 2 * H) dst[c] = c < n[0] ? S.cb[0][c] : S.cb[1][c - n[0]];
+  }
   return true;
 }
 

@@ -560,3 +560,43 @@ def test_read_beyond_the_oversize_limit_is_refused(golden):
     assert e.value.code == -4
     data, offs = csr([big[:200_000]])
     gix.classify(data, offs)
+
+
+@pytest.mark.parametrize("slots", [False, True])
+def test_long_read_tier_at_its_edges(tmp_path, slots):
+    """The long-read tier at its limits: the shortest read it gets (321 bases), the last and first
+    lengths of its half-blocks (1,023 and 1,024 seeds: 15,376 and 15,377 bases), its longest read
+    (20,480) and one past it; on references with a copy, with a segment twice in one reference (two
+    postings of a reference under a seed), and with stray seeds of the matched reference elsewhere
+    (postings out of seed order); forward, reversed, lowercase and with IUPAC letters; chimeras. With
+    both probe layouts; every result equals the oracle's."""
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(71)
+    acgt = np.frombuffer(b"ACGT", np.uint8)
+    comp = np.zeros(256, np.uint8)
+    comp[list(b"ACGTN")] = list(b"TGCAN")
+    core = acgt[rng.integers(0, 4, 30000)]
+    twice = acgt[rng.integers(0, 4, 40000)]
+    twice[30000:36000] = twice[1000:7000]
+    stray = core.copy()
+    for at in range(0, 2000, 40):  # seed windows of the core's far end at its start
+        stray[at:at + 17] = core[20000 + 3 * at:20017 + 3 * at]
+    refs = [core, twice, stray, core[5000:15000].copy(), acgt[rng.integers(0, 4, 9000)]]
+    offs = np.zeros(len(refs) + 1, np.uint64)
+    offs[1:] = np.cumsum([len(r) for r in refs])
+    image = M.build_image(np.concatenate(refs), offs, [f"ref{i}" for i in range(len(refs))])
+    path = tmp_path / "edges.mhm"
+    image.tofile(path)
+    gix, oix = M.Index(image), O.Index(str(path))
+    gix.set_probe_slots(slots)
+    seqs = []
+    for n in (321, 322, 350, 1100, 6000, 15376, 15377, 20479, 20480, 20481):
+        for src in (core, twice, stray):
+            r = src[1000:1000 + n].copy()
+            hit = rng.random(n) < 0.02
+            r[hit] = acgt[rng.integers(0, 4, int(hit.sum()))]
+            seqs += [r.tobytes(), comp[r[::-1]].tobytes()]
+    seqs += [seqs[6].lower(), seqs[8][:500] + b"NNNNRYKM" + seqs[8][508:], seqs[9][:40] + b"U" + seqs[9][41:]]
+    seqs += [core[2000:4000].tobytes() + twice[9000:12000].tobytes(), twice[500:8000].tobytes()]
+    check_against_oracle(gix, oix, seqs)

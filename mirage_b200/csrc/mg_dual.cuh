@@ -1,4 +1,5 @@
-// Dual-strand warp path: both strands of a read at once, one half-warp per strand (lanes 0-15
+// Dual-strand warp path: reads that match at most one reference per strand go through registers
+// (single_ref_strands); the others, both strands at once, one half-warp per strand (lanes 0-15
 // the forward strand, lanes 16-31 its reverse complement), for reads of up to kLeanQ bases with
 // at most 64 postings per strand.
 //
@@ -31,7 +32,8 @@ struct alignas(16) DualSmemT {  // 16-byte aligned: the table clear stores 16 by
                                 // records' refID, first-seed position and last-seed end
   uint32_t t[2][2][Cap];          // occurrence table (ref key, found mask, then occMax); from the
                                 // diagonal runs on: the records' seed indices and segmax
-  uint8_t q[2][kLeanQ];         // strand bases: forward, reverse complement
+  alignas(4) uint8_t q[2][kLeanQ + 12];  // strand bases (load_strands): forward, from 4 + the read's
+                                       // address modulo 4; reverse complement, from 0
 };
 using DualSmem = DualSmemT<64>;  // the first dual tier, over every read
 
@@ -45,16 +47,15 @@ __device__ __forceinline__ unsigned long long below64(int i) {  // bits 0..i-1
 // Bits of a full-warp ballot that belong to this lane's half.
 __device__ __forceinline__ uint32_t half_bits(uint32_t ballot, int sh) { return (ballot >> sh) & 0xFFFFu; }
 
-// Both strands of one read (bases already in S.q). Warp-uniform return: kStrandOk, or
+// Both strands of one read (q: this half's bases in S.q). Warp-uniform return: kStrandOk, or
 // kStrandOverflow when either strand does not fit. Each lane receives its half's strand result:
 // *n_out run records (step 5) in S.c[half][0..2] and S.t[half][0], in ascending refID.
 template <int Cap>
-__device__ int dual_strands(const DevIndex& ix, uint32_t L, DualSmemT<Cap>& S, uint32_t* n_out) {
+__device__ int dual_strands(const DevIndex& ix, uint32_t L, DualSmemT<Cap>& S, const uint8_t* q, uint32_t* n_out) {
   const unsigned FULL = 0xffffffffu;
   const uint32_t EMPTY = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31, half = lane >> 4, hl = lane & 15, sh = half * 16;
   const uint32_t k = (uint32_t)ix.k, step = (uint32_t)ix.step;
-  const uint8_t* q = S.q[half];
   uint32_t* e_ref = S.a[half][0];
   uint32_t* e_pos = S.a[half][1];
   uint32_t* e_fj = S.a[half][2];
@@ -300,6 +301,176 @@ __device__ int dual_strands(const DevIndex& ix, uint32_t L, DualSmemT<Cap>& S, u
   return kStrandOk;
 }
 
+// The read's strands into S.q, a word at a time: the aligned words of the read (bytes beside it in
+// the first and the last do no harm) in upper case, then the reverse complement's words from them.
+// A read with a byte outside ACGT (or with such a neighbour in those words) goes byte by byte through
+// comp, the table of complement(upper(byte)). false: a byte without a complement.
+__device__ __forceinline__ bool load_strands(const uint8_t* raw, uint32_t L, uint8_t (*q)[kLeanQ + 12], const uint8_t* comp) {
+  const unsigned FULL = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31, o = (uint32_t)(uintptr_t)raw & 3u;
+  const uint32_t* g = (const uint32_t*)((uintptr_t)raw & ~(uintptr_t)3);
+  uint32_t* w0 = reinterpret_cast<uint32_t*>(q[0]) + 1;
+  uint32_t* w1 = reinterpret_cast<uint32_t*>(q[1]);
+  const uint32_t nw = L ? (o + L + 3) >> 2 : 0u;
+  bool ok = true;
+  for (uint32_t i = lane; i < nw; i += 32) {
+    const uint32_t u = upper4(__ldg(g + i));
+    ok = ok && acgt4(u);
+    w0[i] = u;
+  }
+  if (__all_sync(FULL, ok)) {
+    __syncwarp();
+    for (uint32_t i = lane; 4 * i < L; i += 32) {  // bases 4 i .. 4 i + 3: the bytes x .. x + 3 of q[0], reversed
+      const uint32_t x = 4 + o + L - 4 - 4 * i;  // at least 1: up to three bytes before the read, not used
+      const uint32_t* wx = reinterpret_cast<const uint32_t*>(q[0]) + (x >> 2);
+      w1[i] = comp4(__byte_perm(__funnelshift_r(wx[0], wx[1], 8 * (x & 3u)), 0, 0x0123));
+    }
+    __syncwarp();
+    return true;
+  }
+  bool bad = false;
+  for (uint32_t i = lane; i < L; i += 32) {
+    q[0][4 + o + i] = upper_dev(raw[i]);
+    const uint8_t c = comp[raw[L - 1 - i]];
+    bad |= c == 0;
+    q[1][i] = c;
+  }
+  bad = __any_sync(FULL, bad);
+  return !bad;
+}
+
+// Both strands of a read in registers, for the read that most are: on each strand at most one
+// reference with postings under two found seeds in a row (a link: without one a reference has no
+// occurrence run of 2, so no diagonal run of 2, so it is no candidate, and a strand without links
+// has none; Analyser.cpp:2057-2115, 2337-2402), at most one posting of it under a seed, its positions
+// ascending with the seeds, and no bucket beyond a slot's kSlotPosts. Then that reference is kept
+// whatever the other references' runs, its postings in seed order are in sorted order, and the runs
+// are ballots. A seed per lane: half-warps side by side for up to 16 seeds, else the warp takes the
+// strands in turn. Anything else returns false, for dual_strands, which costs such a read about a
+// hundred instructions more than before; of reads that match one reference of a large set that is
+// about one in fifty. The table, compaction and rank sort of dual_strands were most of the 1,091 warp
+// instructions of a read of 75-300 bases, which issue bound; 607 are left, and the kernel takes 831 us
+// per 1 M such reads on 5,000 references (1,312 us before), 209 us per 200,000 reads of 250 bases on
+// references that share repeats (313 us before). Bound now by issue (60% of the slots) and by the
+// slots' random DRAM sectors (70% of the measured gather rate) together. Measured and not kept: the
+// next reads' offsets and bases asked for a chunk ahead (859 us), 32-byte slot loads (827 us).
+// The records as dual_strands leaves them; n0 and n1 of them on the two strands.
+template <int Cap>
+__device__ __forceinline__ bool single_ref_strands(const DevIndex& ix, uint32_t L, DualSmemT<Cap>& S, const uint8_t* q0,
+                                                   uint32_t* n0, uint32_t* n1) {
+  const unsigned FULL = 0xffffffffu;
+  constexpr uint32_t kNoRef = 0xFFFFFFFFu, kNoPrev = 0xFFFFFFFEu;  // references are below 2^32 - 2
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t k = (uint32_t)ix.k, step = (uint32_t)ix.step;
+  *n0 = *n1 = 0;
+  if (L <= k) return true;
+  const uint32_t ns = (L - k + step - 1) / step;
+  if (ns > 32) return false;
+  const bool wide = ns > 16;  // warp-uniform, as everything above
+  const uint32_t hl = wide ? lane : lane & 15u, sh = lane - hl, wm = wide ? FULL : 0xFFFFu;
+  const uint32_t below = (1u << hl) - 1u;
+  for (int pass = 0; pass <= (wide ? 1 : 0); pass++) {
+    const uint32_t strand = wide ? (uint32_t)pass : lane >> 4;
+    const uint8_t* q = strand ? S.q[1] : q0;
+    uint32_t cnt = 0, r[kSlotPosts], p[kSlotPosts];
+    bool found = false;
+    if (hl < ns) {
+      const uint32_t h = hash28_dev(q + hl * step, ix.hlen);
+      if (ix.slots) {
+        const uint4* sl = ix.slots + (size_t)h * kSlotVecs;
+        const uint4 v0 = __ldg(sl), v1 = __ldg(sl + 1);
+        cnt = v0.x;
+        r[0] = v0.z, p[0] = v0.w, r[1] = v1.x, p[1] = v1.y, r[2] = v1.z, p[2] = v1.w;
+        if (cnt > 3) {
+          const uint4 v2 = __ldg(sl + 2), v3 = __ldg(sl + 3);
+          r[3] = v2.x, p[3] = v2.y, r[4] = v2.z, p[4] = v2.w, r[5] = v3.x, p[5] = v3.y, r[6] = v3.z, p[6] = v3.w;
+        }
+      } else {
+        const uint32_t o = __ldg(ix.dir + h);
+        cnt = __ldg(ix.dir + h + 1) - o;
+#pragma unroll
+        for (int t = 0; t < kSlotPosts; t++)
+          if ((uint32_t)t < cnt) {
+            const uint2 v = __ldg(ix.post + o + t);
+            r[t] = v.x;
+            p[t] = v.y;
+          }
+      }
+      found = cnt > 0 || h == ix.empty_hash;
+    }
+    const uint32_t mc = __reduce_max_sync(FULL, cnt);
+    if (mc > (uint32_t)kSlotPosts) return false;
+#pragma unroll
+    for (int t = 0; t < kSlotPosts; t++)
+      if ((uint32_t)t >= cnt) r[t] = kNoRef;
+    // links: this seed's references among those of the found seed before it
+    const uint32_t fb = (__ballot_sync(FULL, found) >> sh) & below;
+    const uint32_t prev = fb ? sh + 31u - __clz(fb) : lane;
+    uint32_t pc = __shfl_sync(FULL, cnt, prev);
+    pc = fb ? pc : 0u;
+    uint32_t lr = kNoRef;
+    bool other = false;  // two references linked
+#pragma unroll
+    for (int t = 0; t < kSlotPosts; t++) {
+      if ((uint32_t)t >= mc) break;  // warp-uniform
+      uint32_t x = __shfl_sync(FULL, r[t], prev);
+      x = (uint32_t)t < pc ? x : kNoPrev;
+      bool eq = r[0] == x;
+#pragma unroll
+      for (int u = 1; u < kSlotPosts; u++)
+        if ((uint32_t)u < mc) eq = eq || r[u] == x;
+      if (eq) {
+        other = other || (lr != kNoRef && lr != x);
+        lr = x;
+      }
+    }
+    const uint32_t lb = __ballot_sync(FULL, lr != kNoRef);
+    if (lb == 0) continue;  // no candidate on either strand (or this one)
+    const uint32_t mine = (lb >> sh) & wm;
+    uint32_t ref = __shfl_sync(FULL, lr, mine ? sh + __ffs(mine) - 1 : lane);
+    ref = mine ? ref : kNoPrev;
+    other = other || (lr != kNoRef && lr != ref);
+    // its posting under each seed
+    uint32_t pos = 0;
+    bool has = false;
+#pragma unroll
+    for (int t = 0; t < kSlotPosts; t++)
+      if ((uint32_t)t < mc && r[t] == ref) {
+        other = other || has;
+        has = true;
+        pos = p[t];
+      }
+    const uint32_t hb = (__ballot_sync(FULL, has) >> sh) & wm, hp = hb & below;
+    const uint32_t before = hp ? 31u - __clz(hp) : 0u;
+    const uint32_t pp = __shfl_sync(FULL, pos, hp ? sh + before : lane);
+    other = other || (has && hp && pp > pos);
+    if (__any_sync(FULL, other)) return false;
+    // runs: cb marks the seeds that continue the run of the seed before them
+    const bool cont = has && hp && before + 1 == hl && (uint64_t)pp + step == pos;
+    const uint32_t cb = (__ballot_sync(FULL, cont) >> sh) & wm;
+    const bool end = has && cb && !((cb >> 1 >> hl) & 1u);  // no run of 2: no candidate (:2402)
+    const uint32_t starts = hb & ~cb & (below | (1u << hl));
+    const uint32_t first = starts ? 31u - __clz(starts) : 0u;
+    const uint32_t sr = __shfl_sync(FULL, pos, sh + first);
+    const uint32_t eb = __ballot_sync(FULL, end);
+    if (end) {
+      const uint32_t at = __popc((eb >> sh) & below);
+      S.c[strand][0][at] = ref;
+      S.c[strand][1][at] = sr;
+      S.c[strand][2][at] = pos + step;
+      S.t[strand][0][at] = first | (hl << 8);
+    }
+    if (wide) {
+      (pass ? *n1 : *n0) = __popc(eb);
+    } else {
+      *n0 = __popc(eb & 0xFFFFu);
+      *n1 = __popc(eb >> 16);
+    }
+  }
+  __syncwarp();
+  return true;
+}
+
 // Read r on the dual path; false when it does not fit (the caller hands it on).
 // comp: the block's 256-entry table of complement(upper(byte)), 0 where there is none.
 // The read's run records (forward strand first) go to its staging slots, or to the arena when
@@ -316,14 +487,7 @@ __device__ bool process_read_dual(const DevIndex& ix, const BatchDev& b, uint32_
   if (Lr > (uint64_t)kLeanQ) return false;
   const uint32_t L = (uint32_t)Lr;
   const uint8_t* raw = b.bases + o0;
-  uint32_t badl = 0;
-  for (uint32_t i = lane; i < L; i += 32) {
-    S.q[0][i] = upper_dev(raw[i]);
-    const uint8_t c = comp[raw[L - 1 - i]];
-    badl |= c == 0;
-    S.q[1][i] = c;
-  }
-  if (__any_sync(FULL, badl)) {
+  if (!load_strands(raw, L, S.q, comp)) {
     if (lane == 0)
       b.reads[r] = mg_read_result{-1.0f, 0, 0, 0, MG_READ_BAD_BYTE, 0, 0};
     if (lane == 0) atomicOr(errw, kErrBadInput);
@@ -331,9 +495,15 @@ __device__ bool process_read_dual(const DevIndex& ix, const BatchDev& b, uint32_
     return true;
   }
   __syncwarp();
-  uint32_t nh;
-  if (dual_strands(ix, L, S, &nh) != kStrandOk) return false;
-  const uint32_t n0 = __shfl_sync(FULL, nh, 0), n1 = __shfl_sync(FULL, nh, 16), tot = n0 + n1;
+  const uint8_t* q0 = S.q[0] + 4 + ((uint32_t)(uintptr_t)raw & 3u);
+  uint32_t n0, n1;
+  if (Cap != 64 || !single_ref_strands(ix, L, S, q0, &n0, &n1)) {
+    uint32_t nh;
+    if (dual_strands(ix, L, S, lane < 16 ? q0 : S.q[1], &nh) != kStrandOk) return false;
+    n0 = __shfl_sync(FULL, nh, 0);
+    n1 = __shfl_sync(FULL, nh, 16);
+  }
+  const uint32_t tot = n0 + n1;
   if (tot == 0) {
     if (lane == 0) b.reads[r] = mg_read_result{-1.0f, 0, 0, 0, 0, 0, 0};
     __syncwarp();

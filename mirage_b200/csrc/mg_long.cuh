@@ -92,21 +92,6 @@ __device__ __forceinline__ void lg_sync(int bar, uint32_t G) {
   asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(G) : "memory");
 }
 
-// upper_dev on each byte of w: bytes 0x61..0x7F lose 0x20.
-__device__ __forceinline__ uint32_t upper4(uint32_t w) {
-  const uint32_t m = (((w & 0x7F7F7F7Fu) + 0x1F1F1F1Fu) & ~w) & 0x80808080u;
-  return w - (m >> 2);
-}
-// Whether all four bytes of w (upper case) are in ACGT: two bits of a byte pick the letter that it
-// has to be.
-__device__ __forceinline__ bool acgt4(uint32_t w) {
-  const uint32_t c = (w >> 1) & 0x03030303u;  // A 0, C 1, T 2, G 3
-  const uint32_t t = c | (c >> 4);
-  return __byte_perm(0x47544341u, 0, (t & 0xFFu) | ((t >> 8) & 0xFF00u)) == w;
-}
-// Complement of four ACGT bytes: A and T differ in 0x15, C and G (bit 1 set) in 0x04.
-__device__ __forceinline__ uint32_t comp4(uint32_t w) { return w ^ 0x15151515u ^ (((w >> 1) & 0x01010101u) * 0x11u); }
-
 // hash28_dev of the 17-byte window a..a+16 of an ACGT read in upper case (strand 0), or of its
 // reverse complement (strand 1). The five aligned words loaded each hold a byte of the window
 // ((a & 3) + 17 <= 20).

@@ -600,3 +600,54 @@ def test_long_read_tier_at_its_edges(tmp_path, slots):
     seqs += [seqs[6].lower(), seqs[8][:500] + b"NNNNRYKM" + seqs[8][508:], seqs[9][:40] + b"U" + seqs[9][41:]]
     seqs += [core[2000:4000].tobytes() + twice[9000:12000].tobytes(), twice[500:8000].tobytes()]
     check_against_oracle(gix, oix, seqs)
+
+
+@pytest.mark.parametrize("slots", [False, True])
+def test_strands_in_registers_and_their_hand_offs(tmp_path, slots):
+    """The first dual-strand tier's form for reads with one linked reference per strand, and the reads
+    that it leaves to the general form: 16 and 17 seeds (271 and 272 bases) and the longest (320), a
+    seed's bucket of 7 and of 8 postings (copies of a window elsewhere), a reference twice under a
+    seed, its positions out of seed order, two references, one linked reference on each strand, links
+    without a diagonal run, no seed at all, lowercase, IUPAC letters in the read and beside it, and
+    every address modulo 4. With both probe layouts; every result equals the oracle's."""
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(73)
+    acgt = np.frombuffer(b"ACGT", np.uint8)
+    comp = np.zeros(256, np.uint8)
+    comp[list(b"ACGTN")] = list(b"TGCAN")
+    core = acgt[rng.integers(0, 4, 12000)]
+    other = acgt[rng.integers(0, 4, 9000)]
+    other[2000:2400] = core[3000:3400]             # two references
+    other[5000:5200] = comp[core[6000:6200][::-1]]  # one on each strand
+    twice = acgt[rng.integers(0, 4, 9000)]
+    twice[1000:1300] = other[7000:7300]
+    twice[4000:4300] = other[7000:7300]            # a reference twice under a seed
+    swapped = acgt[rng.integers(0, 4, 6000)]
+    for j in range(8):                             # windows of core[9000:] in reverse order
+        swapped[3000 - 40 * j:3017 - 40 * j] = core[9000 + 15 * j:9017 + 15 * j]
+    many = [acgt[rng.integers(0, 4, 400)] for _ in range(7)]
+    for i, m in enumerate(many):                   # a window in 7 and one in 8 references
+        m[100:117] = core[10030:10047]
+        if i < 6:
+            m[200:217] = core[11030:11047]
+    refs = [core, other, twice, swapped] + many
+    offs = np.zeros(len(refs) + 1, np.uint64)
+    offs[1:] = np.cumsum([len(r) for r in refs])
+    image = M.build_image(np.concatenate(refs), offs, [f"ref{i}" for i in range(len(refs))])
+    path = tmp_path / "registers.mhm"
+    image.tofile(path)
+    gix, oix = M.Index(image), O.Index(str(path))
+    gix.set_probe_slots(slots)
+    seqs = []
+    for n in (30, 31, 32, 46, 47, 76, 151, 271, 272, 273, 319, 320):
+        for at in (100, 3050, 6010, 8990, 10000, 11000):
+            r = core[at:at + n].copy()
+            seqs += [r.tobytes(), comp[r[::-1]].tobytes()]
+            hit = rng.random(n) < 0.03
+            r[hit] = acgt[rng.integers(0, 4, int(hit.sum()))]
+            seqs.append(r.tobytes())
+    seqs += [other[7000:7250].tobytes(), twice[990:1240].tobytes(), twice[3990:4301].tobytes(), acgt[rng.integers(0, 4, 200)].tobytes()]
+    seqs += [seqs[40].lower(), b"N" * 60, core[100:200].tobytes() + b"N" + core[201:300].tobytes(), core[400:640].tobytes()]
+    seqs += [core[500:650].tobytes() + core[8000:8100].tobytes(), core[3000:3100].tobytes() + other[2200:2300].tobytes()]
+    check_against_oracle(gix, oix, seqs)

@@ -212,8 +212,8 @@ int mg_build_image_device(int device, const uint8_t* bases, const uint64_t* offs
 
 /* Plain form. Replaces the reference's per-batch sequence TPrepareGPUAnalysis (Analyser.cpp:
  * 1317) -> CPUGetHighestScore (MatrixCPU.cpp:417) -> strand merge (Analyser.cpp:592-611):
- * one block per read in one launch per batch (the global-memory tier takes reads beyond its
- * shared memory), host buffers in and out with synchronous copies.
+ * one block per read in one launch per batch (the long-read and global-memory tiers take reads
+ * beyond its shared memory), host buffers in and out with synchronous copies.
  * Read lengths: like the reference's CPU path, no cap below 2,000,000 bases (the batched forms
  * too; the served form takes up to 65,535). Reads past 65,535 bases, 4,400 seeds or 65,536
  * postings per strand go to the oversize tier, whose device workspace is sized by the first

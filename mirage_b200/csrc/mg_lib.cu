@@ -170,7 +170,7 @@ __device__ __forceinline__ uint32_t walk_record(const DevIndex& ix, const uint8_
 // is a candidate whose Score, percentage and relative score (MatrixCPU.cpp:18-214,
 // MatrixResult.cpp:21-29) replace its records, compacted in place; then the strand merge and top
 // group as write_read_result_s (Analyser.cpp:592-611, 388).
-__global__ void __launch_bounds__(kFinThreads) k_finish_dual(DevIndex ix, BatchDev b, StageDev sd) {
+__global__ void __launch_bounds__(kFinThreads) k_finish_dual(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd) {
   const unsigned FULL = 0xffffffffu;
   __shared__ uint8_t comp[256];
   __shared__ uint32_t covs[kFinThreads * kCovStride];
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(Warps * 32) k_classify_dual_list(DevIndex ix, 
 // Long-read tier over the dual tiers' leftovers and the plain form's, a block per read with work
 // stealing (the next read is taken while this one is classified); its own leftovers go to the
 // global-memory tier.
-__global__ void __launch_bounds__(2 * LongSmem::H, 4) k_classify_long(DevIndex ix, BatchDev b, StageDev sd,
+__global__ void __launch_bounds__(2 * LongSmem::H, 4) k_classify_long(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd,
                                                                      const uint32_t* list, const unsigned* list_n,
                                                                      unsigned* cursor, uint32_t* next,
                                                                      unsigned* next_n, unsigned* n_small,
@@ -354,11 +354,25 @@ __global__ void __launch_bounds__(2 * LongSmem::H, 4) k_classify_long(DevIndex i
   }
 }
 
-// Block tier over a list of reads (list == nullptr: every read, the plain form); the reads that
-// do not fit go to the next list, or, from the last tier, are marked for the oversize tier
-// (kErrHuge: the host then runs the batch again with it).
+// Plain form: a block of two warps per read, one launch over the batch; the reads that do not fit go
+// to the long-read tier.
+__global__ void __launch_bounds__(2 * PlainSmem::H) k_classify_plain(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd, uint32_t* next,
+                                                                    unsigned* next_n) {
+  __shared__ PlainSmem S;
+  for (int c = threadIdx.x; c < 256; c += blockDim.x) S.comp[c] = complement_dev(upper_dev((uint8_t)c));
+  if (threadIdx.x == 0) S.handed = 0;
+  __syncthreads();
+  const uint32_t r = blockIdx.x;
+  if (!process_read_long(ix, b, r, S, sd.stage, sd.arena, sd.arena_cap, sd.arena_n, b.err, nullptr, nullptr)) {
+    if (threadIdx.x == 0) next[atomicAdd(next_n, 1u)] = r;
+  }
+}
+
+// Block and global tiers over a list of reads; the reads that do not fit go to the next list, or,
+// from the last tier, are marked for the oversize tier (kErrHuge: the host then runs the batch again
+// with it).
 template <int G>
-__global__ void __launch_bounds__(G) k_classify_block(DevIndex ix, BatchDev b, StageDev sd, const uint32_t* list,
+__global__ void __launch_bounds__(G) k_classify_block(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd, const uint32_t* list,
                                                        const unsigned* list_n, unsigned* cursor, uint32_t* next,
                                                        unsigned* next_n, uint8_t* gws, WsLayout lay, Caps caps,
                                                        int last_tier) {
@@ -367,15 +381,14 @@ __global__ void __launch_bounds__(G) k_classify_block(DevIndex ix, BatchDev b, S
   uint8_t* base = gws ? gws + (size_t)blockIdx.x * lay.total : dsm;
   const StrandWS ws = ws_from(base, lay, caps.c);
   RedTmp<G>* red = (RedTmp<G>*)(base + lay.red);
-  const uint64_t n = list ? (uint64_t)*list_n : b.n;
+  const uint32_t n = *list_n;
   for (;;) {
-    if (threadIdx.x == 0) s_item = cursor ? atomicAdd(cursor, 1u) : 0xFFFFFFFFu;
+    if (threadIdx.x == 0) s_item = atomicAdd(cursor, 1u);
     __syncthreads();
-    uint64_t item = cursor ? (uint64_t)s_item : (uint64_t)blockIdx.x;
+    const uint32_t item = s_item;
     __syncthreads();
-    if (!cursor && item >= n) break;
     if (item >= n) break;
-    const uint32_t r = list ? list[item] : (uint32_t)item;
+    const uint32_t r = list[item];
     if (!process_read<G>(ix, b, r, ws, caps, red, sd.stage, sd.arena, sd.arena_cap, sd.arena_n, b.err)) {
       if (threadIdx.x == 0) {
         if (last_tier) {
@@ -387,7 +400,6 @@ __global__ void __launch_bounds__(G) k_classify_block(DevIndex ix, BatchDev b, S
       }
     }
     __syncthreads();
-    if (!cursor) break;
   }
 }
 
@@ -425,7 +437,7 @@ __device__ void read_need(const DevIndex& ix, const uint8_t* raw, uint32_t L, Re
 // kErrHuge, so that the host grows the slabs and runs the batch again; a read beyond the hard
 // limits, or with more than 65,535 candidates on a strand, is refused (kErrLimit).
 template <int G>
-__global__ void __launch_bounds__(G) k_classify_huge(DevIndex ix, BatchDev b, StageDev sd, const uint32_t* list,
+__global__ void __launch_bounds__(G) k_classify_huge(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd, const uint32_t* list,
                                                       const unsigned* list_n, unsigned* cursor, uint8_t* hws,
                                                       WsLayout lay, Caps caps, unsigned* need) {
   __shared__ uint32_t s_item;
@@ -718,7 +730,7 @@ __global__ void k_log_probe(uint32_t lo_bits, uint32_t n, float* out) {
   if (i < n) out[i] = log_dev_raw(__uint_as_float(lo_bits + i));
 }
 
-__global__ void k_eval_logf(DevIndex ix, const float* x, float* out, uint64_t n, int* errw) {
+__global__ void k_eval_logf(const __grid_constant__ DevIndex ix, const float* x, float* out, uint64_t n, int* errw) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int err = 0;
@@ -728,7 +740,7 @@ __global__ void k_eval_logf(DevIndex ix, const float* x, float* out, uint64_t n,
 
 // Scoring-only drop-in (MatrixCPU::CPUGetHighestScore): one thread per candidate, like the
 // reference's CUDA kernel, with the semantics of CalculateScore.
-__global__ void k_score_candidates(DevIndex ix, uint64_t n_strands, const uint64_t* q_off, const uint8_t* bases,
+__global__ void k_score_candidates(const __grid_constant__ DevIndex ix, uint64_t n_strands, const uint64_t* q_off, const uint8_t* bases,
                                    const uint64_t* c_off, const uint32_t* cand_ref, const uint64_t* r_off,
                                    const uint32_t* runs, uint64_t n_cands, const uint64_t* cand_strand,
                                    float* score_out, float* pct_out, float* rel_out, uint32_t* hit_ws,
@@ -784,7 +796,7 @@ namespace mg {
 // they differ, so that the device reproduces the reference's logf bit for bit.
 // log_den[lm] = the denominator of relative_score at len_max = lm (its own code, so the values are
 // the ones relative_score computes).
-__global__ void k_fill_log_den(DevIndex ix, float* out) {
+__global__ void k_fill_log_den(const __grid_constant__ DevIndex ix, float* out) {
   const uint32_t lm = blockIdx.x * blockDim.x + threadIdx.x;
   if (lm > 0xFFFFu) return;
   const double l = (double)__uint2float_rn(lm);
@@ -1173,7 +1185,18 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
     // timing events (start, end) per tier: ev[0..1] first tier, ev[2..3] nothing,
     // ev[3..4] long-read tier, ev[4..5] global tier, ev[6..7] compaction
     if (tm) CU(cudaEventRecord(ix->ev[0], st));
-    auto global_tier = [&](cudaStream_t s) {
+    const Shapes sh = shapes(ix);
+    // the tiers behind the dual-strand ones and the plain form's kernel, on stream s
+    auto further_tiers = [&](cudaStream_t s) -> int {
+      if (tm) CU(cudaEventRecord(ix->ev[2], s));
+      if (tm) CU(cudaEventRecord(ix->ev[3], s));
+      if (ix->dix.n_refs <= (1u << 21))
+        k_classify_long<<<sh.long_blocks_per_sm * sms, 2 * LongSmem::H, sizeof(LongSmem), s>>>(
+            ix->dix, b, sd, b.ovf0b, b.n_ovf0b, work_long, b.ovf2, b.n_ovf2, n_small, n_large);
+      else
+        k_classify_block<kB2Threads><<<(unsigned)sms, kB2Threads, l2.total, s>>>(
+            ix->dix, b, sd, b.ovf0b, b.n_ovf0b, b.work2, b.ovf2, b.n_ovf2, nullptr, l2, c2, 0);
+      if (tm) CU(cudaEventRecord(ix->ev[4], s));
       k_classify_block<kB3Threads><<<kB3Blocks, kB3Threads, 0, s>>>(ix->dix, b, sd, b.ovf2, b.n_ovf2, b.work3, ovf3,
                                                                     n_ovf3, w.gws.as<uint8_t>(), l3, c3, !w.hmode);
       // the oversize tier, once a batch of this workspace has needed it: one block while it has
@@ -1181,26 +1204,20 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
       if (w.hmode)
         k_classify_huge<kHugeThreads><<<(unsigned)std::max(1, w.hslabs), kHugeThreads, 0, s>>>(
             ix->dix, b, sd, ovf3, n_ovf3, work4, w.hslabs ? w.hws.as<uint8_t>() : nullptr, lh, ch, huge_need);
+      if (tm) CU(cudaEventRecord(ix->ev[5], s));
+      return MG_OK;
     };
     if (plain) {
-      // every read gets its own block (one launch for the batch)
-      k_classify_block<kB2Threads><<<(unsigned)n, kB2Threads, l2.total, st>>>(
-          ix->dix, b, sd, nullptr, nullptr, nullptr, b.ovf2, b.n_ovf2, nullptr, l2, c2, 0);
-      if (tm) {
-        CU(cudaEventRecord(ix->ev[1], st));
-        CU(cudaEventRecord(ix->ev[2], st));
-        CU(cudaEventRecord(ix->ev[3], st));
-        CU(cudaEventRecord(ix->ev[4], st));
-      }
-      global_tier(st);
-      if (tm) CU(cudaEventRecord(ix->ev[5], st));
+      k_classify_plain<<<(unsigned)n, 2 * PlainSmem::H, 0, st>>>(ix->dix, b, sd, b.ovf0b, b.n_ovf0b);
+      if (tm) CU(cudaEventRecord(ix->ev[1], st));
+      const int rc = further_tiers(st);
+      if (rc) return rc;
     } else {
       if (!w.side) {
         CU(cudaStreamCreateWithFlags(&w.side, cudaStreamNonBlocking));
         CU(cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming));
         CU(cudaEventCreateWithFlags(&w.join, cudaEventDisableTiming));
       }
-      const Shapes sh = shapes(ix);
       if (sh.first_tier == 1)
         k_classify_dual<<<sh.dual_blocks_per_sm * sms, kW1Warps * 32, 0, st>>>(ix->dix, b, sd, sh.steal_chunk);
       // tiers of 64, 128 and 256 postings per strand, each over the one before's leftovers
@@ -1213,17 +1230,8 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
       // the dual tier's finishing pass (different reads, disjoint slots; arena space by atomics)
       CU(cudaEventRecord(w.fork, st));
       CU(cudaStreamWaitEvent(w.side, w.fork, 0));
-      if (tm) CU(cudaEventRecord(ix->ev[2], w.side));
-      if (tm) CU(cudaEventRecord(ix->ev[3], w.side));
-      if (ix->dix.n_refs <= (1u << 21))
-        k_classify_long<<<sh.long_blocks_per_sm * sms, 2 * LongSmem::H, sizeof(LongSmem), w.side>>>(
-            ix->dix, b, sd, b.ovf0b, b.n_ovf0b, work_long, b.ovf2, b.n_ovf2, n_small, n_large);
-      else
-        k_classify_block<kB2Threads><<<(unsigned)sms, kB2Threads, l2.total, w.side>>>(
-            ix->dix, b, sd, b.ovf0b, b.n_ovf0b, b.work2, b.ovf2, b.n_ovf2, nullptr, l2, c2, 0);
-      if (tm) CU(cudaEventRecord(ix->ev[4], w.side));
-      global_tier(w.side);
-      if (tm) CU(cudaEventRecord(ix->ev[5], w.side));
+      const int rc = further_tiers(w.side);
+      if (rc) return rc;
       CU(cudaEventRecord(w.join, w.side));
       k_finish_dual<<<(unsigned)std::min<uint64_t>((n + kFinThreads - 1) / kFinThreads,
                                                    (uint64_t)sms * sh.finish_blocks_per_sm),

@@ -80,16 +80,28 @@ struct alignas(16) LongSm {
 };
 
 // The classes of reads: the batched forms' tier (reads to 20,480 bases and 4,096 postings per strand)
-// with four blocks per SM, and the plain form's first kernel, one block of two warps per read.
+// with four blocks per SM, and the plain form's kernel, one block of two warps per read, up to 15 per
+// SM (11,000 reads of 150 bases: 97 us; a block of 256 threads per read with two bitonic sorts per
+// strand, the form before, 1,010 us; room for 256 postings instead of 512 makes no difference).
 using LongSmem = LongSm<128, 2048, 1023, 256, 96>;
+using PlainSmem = LongSm<32, 512, 255, 64, 32>;
 constexpr uint32_t kLgQ = 20480;
 static_assert(4 * (sizeof(LongSmem) + 1024) <= 233472, "four blocks per SM");
 
 __device__ __forceinline__ uint32_t lg_mix(uint32_t x) { return (x * 2654435761u) ^ (x >> 15); }
 
-// Barrier over the G threads of a group (a named barrier: 1 + half for a half, 0 for the block).
-__device__ __forceinline__ void lg_sync(int bar, uint32_t G) {
-  asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(G) : "memory");
+// Barrier over a group: the block (bar 0), or half bar - 1 of H threads. The ids are immediates: with
+// an id in a register a block is given all 16 barriers, and four blocks fill the SM.
+template <int H>
+__device__ __forceinline__ void lg_sync(int bar) {
+  if (bar == 0)
+    asm volatile("bar.sync 0;" ::: "memory");
+  else if (H == 32)
+    __syncwarp();
+  else if (bar == 1)
+    asm volatile("bar.sync 1, %0;" ::"n"(H) : "memory");
+  else
+    asm volatile("bar.sync 2, %0;" ::"n"(H) : "memory");
 }
 
 // hash28_dev of the 17-byte window a..a+16 of an ACGT read in upper case (strand 0), or of its
@@ -331,7 +343,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
       if (lane == 0 && (j >> 5) < kNW) fm[j >> 5] = fb;
     }
   }
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   uint32_t ne = 0;
   {
     const uint32_t C = (ns + G - 1) / G, lo = min(tid * C, ns), hi = min(lo + C, ns);  // consecutive seeds
@@ -361,7 +373,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
       if (2 * lane < nw) fp[2 * lane] = (uint16_t)(f - c0 - c1);
       if (2 * lane + 1 < nw) fp[2 * lane + 1] = (uint16_t)(f - c1);
     }
-    lg_sync(bar, G);
+    lg_sync<SM::H>(bar);
     uint32_t at = x - own, work = 0, any = 0;
 #pragma unroll 1
     for (uint32_t w = 0; w < kW; w++) {
@@ -381,7 +393,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     if (tid == 0) st[ns] = (uint16_t)ne;
     more = any >> 31;
   }
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   if (ix.slots)
 #pragma unroll 1
     for (uint32_t j = tid; j < ns; j += G) {
@@ -443,7 +455,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
         }
     }
   }
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   const uint32_t fw = (ns - 1) >> 5;
   const uint32_t nf = fp[fw] + __popc(fm[fw]), nfw = (nf + 31) >> 5;
   // 2. the linked references (the warps reconverge between the two searches)
@@ -491,7 +503,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     }
     __syncwarp();
   }
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   const uint32_t R = S.n_rt[half];
   if (R == 0) return kStrandOk;  // no reference at two found seeds in a row: no candidate
   // the bitmaps (R of nfw words) and, behind them, the ones before each word (R nfw half-words) lie over sx
@@ -504,7 +516,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
 #pragma unroll 1
   for (uint32_t i = tid; i < R * nfw; i += G) bm[i] = 0;
   if (tid == 0) S.dup[half] = 0;
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   const uint32_t only = iref[0];
 #pragma unroll 1
   for (uint32_t i0 = 0; i0 < ne; i0 += G) {
@@ -531,7 +543,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
       }
     }
   }
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   if (nfw == 1) {
 #pragma unroll 1
     for (uint32_t id = tid; id < R; id += G) {
@@ -550,7 +562,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
       }
     }
   }
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   uint32_t hs = 0;
 #pragma unroll 1
   for (uint32_t id = lane; id < R; id += 32) hs = max(hs, (uint32_t)best[id]);
@@ -574,7 +586,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   }
 #pragma unroll 1
   for (uint32_t i = tid; i < kRM; i += G) T.segmax[i] = 0;
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   auto rank_of = [&](uint32_t x) -> uint32_t { return T.rk[(x >> 11) & 127u]; };  // of a linked posting
   // 4. the kept postings in (refID, position, seed) order, as indices in sx[0 .. T2)
   auto key_of = [&](uint32_t i) { return ((uint64_t)ps[i] << 11) | (rs[i] & 2047u); };
@@ -603,16 +615,16 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   if (dup) {  // a reference twice under a seed: the postings are counted one by one
 #pragma unroll 1
     for (uint32_t id = tid; id < R; id += G) bfill[id] = 0;
-    lg_sync(bar, G);
+    lg_sync<SM::H>(bar);
 #pragma unroll 1
     for (uint32_t i = tid; i < ne; i += G) {  // a posting's place in its range goes beside its id
       const uint32_t x = rs[i];
       if ((x >> 11) != kNoId && rank_of(x) != kNoId) rs[i] = x | (atomicAdd(&bfill[x >> 11], 1u) << 18);
     }
-    lg_sync(bar, G);
+    lg_sync<SM::H>(bar);
 #pragma unroll 1
     for (uint32_t id = tid; id < R; id += G) T.cnt[id] = (uint16_t)bfill[id];
-    lg_sync(bar, G);
+    lg_sync<SM::H>(bar);
   }
   uint32_t bmax = 0;
 #pragma unroll 1
@@ -630,7 +642,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   if (T2 > kE / 2) return kStrandOverflow;  // group-uniform
   if (tid == 0) boff[nk] = (uint16_t)T2;
   if (tid < (kRM + 31) / 32) badr[tid] = 0;
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
 #pragma unroll 1
   for (uint32_t i = tid; i < ne; i += G) {  // into the ranges, in seed order unless dup
     const uint32_t x = rs[i], id = (x >> 11) & 127u;
@@ -645,7 +657,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     }
     kl[boff[b] + at] = (uint16_t)i;
   }
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   bool bad = dup;  // seed order is not position order: a stray hit, or copies within the reference
 #pragma unroll 1
   for (uint32_t i = tid; i < T2; i += G) {
@@ -662,7 +674,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   }
   bad = __any_sync(FULL, bad);
   if (lane == 0) red[1][warp] = bad;
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   uint32_t any = 0;
 #pragma unroll 1
   for (uint32_t w = 0; w < kW; w++) any |= red[1][w];
@@ -672,7 +684,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     for (uint32_t b = warp; b < nk; b += kW)
       if (dup || ((badr[b >> 5] >> (b & 31u)) & 1u)) rank_range(kl, sx, boff[b], boff[b + 1]);
     sorted = true;
-    lg_sync(bar, G);
+    lg_sync<SM::H>(bar);
   }
   if (!sorted) {  // a reference with many postings out of order: bitonic sort of the indices
     uint32_t N = 2;
@@ -680,7 +692,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     while (N < T2) N <<= 1;
 #pragma unroll 1
     for (uint32_t i = T2 + tid; i < N; i += G) sx[i] = 0xFFFFu;
-    lg_sync(bar, G);
+    lg_sync<SM::H>(bar);
 #pragma unroll 1
     for (uint32_t kk = 2; kk <= N; kk <<= 1) {
 #pragma unroll 1
@@ -701,7 +713,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
             sx[p] = (uint16_t)a;
           }
         }
-        lg_sync(bar, G);
+        lg_sync<SM::H>(bar);
       }
     }
   }
@@ -719,7 +731,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     const uint32_t w = __ballot_sync(FULL, start);
     if (lane == 0 && (i0 + warp * 32) < T2) bk[(i0 >> 5) + warp] = w;
   }
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   auto run_end = [&](uint32_t i) { return i + 1 == T2 || ((bk[(i + 1) >> 5] >> ((i + 1) & 31u)) & 1u); };
   auto run_first = [&](uint32_t i) {  // bit 0 is set: the search ends there at the latest
     uint32_t w = i >> 5, m = bk[w] & (0xFFFFFFFFu >> (31u - (i & 31u)));
@@ -731,7 +743,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
 #pragma unroll 1
   for (uint32_t i = tid; i < T2; i += G)
     if (run_end(i)) atomicMax(&T.segmax[rank_of(rs[sx[i]])], i - run_first(i) + 1);
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   uint32_t M = 0;
 #pragma unroll 1
   for (uint32_t b = lane; b < nk; b += 32) M = max(M, T.segmax[b]);
@@ -779,14 +791,14 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     at = __shfl_sync(FULL, at, 0);
     if (end) kl[at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)i;
   }
-  lg_sync(bar, G);  // every warp has its masks: segmax holds the covered bases from here on
+  lg_sync<SM::H>(bar);  // every warp has its masks: segmax holds the covered bases from here on
   const uint32_t n_ends = S.n_ends[half];
 #pragma unroll 1
   for (uint32_t c0 = 0; c0 < nc; c0 += per) {
     const uint32_t cn = min(per, nc - c0);
 #pragma unroll 1
     for (uint32_t i = tid; i < cn * nw; i += G) cov[i] = 0;
-    lg_sync(bar, G);
+    lg_sync<SM::H>(bar);
 #pragma unroll 1
     for (uint32_t t0 = 0; t0 < n_ends; t0 += G) {
       const uint32_t t = t0 + tid;
@@ -817,7 +829,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
         atomicOr(&cv[wd], (n == 32 ? 0xFFFFFFFFu : ((1u << n) - 1u)) << (lo - w0));
       }
     }
-    lg_sync(bar, G);
+    lg_sync<SM::H>(bar);
 #pragma unroll 1
     for (uint32_t c = warp; c < cn; c += kW) {
       uint32_t hits = 0;
@@ -826,7 +838,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
       hits = __reduce_add_sync(FULL, hits);
       if (lane == 0) T.segmax[c0 + c] = hits;
     }
-    lg_sync(bar, G);
+    lg_sync<SM::H>(bar);
   }
   // 7. scores, a lane per candidate (MatrixCPU.cpp:18-214); one whose runs all fell short of k keeps
   //    Score -2 and is not scored
@@ -865,7 +877,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
       S.hi[half] = hi;
     }
   }
-  lg_sync(bar, G);
+  lg_sync<SM::H>(bar);
   *n_out = S.n_out[half];
   *highest = S.hi[half];
   return kStrandOk;

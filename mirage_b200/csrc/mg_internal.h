@@ -41,6 +41,16 @@ struct DevBuf {
   }
 };
 
+// A piece of a device buffer, by its offset.
+struct DevPiece {
+  uint8_t* p = nullptr;
+  uint64_t at = 0;
+  template <class T>
+  T* as() const {
+    return (T*)p;
+  }
+};
+
 // Device buffers of one classification call in flight (a call owns one at a time).
 struct Workspace {
   DevBuf offs, bases, reads, stage, arena, cands, ctr, ovf, sums, gws, chain;
@@ -121,6 +131,7 @@ struct mg_index {
   mg::MhmIndex host;  // refs, headers, taxids kept; postings released after upload
   mg::DevBuf dir, post, slots, bases, ref_off, ref_len, logx_bitmap, logx_keys, logx_vals, log_den;
   mg::Workspace ws;   // workspace of the synchronous entry points
+  mg::DevBuf score_ws;  // mg_score_candidates' device buffers (under mu)
   cudaStream_t stream = nullptr;
   // chunked batched form: copy streams and per-chunk events (made on first use)
   static constexpr int kMaxChunks = 8;

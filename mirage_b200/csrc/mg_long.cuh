@@ -29,8 +29,8 @@
 // eight strands in flight per SM (issue slots 27% used, DRAM 1.3 TB/s). Measured on a B200 against the
 // form before it (two sizes of block, one strand at a time on 256 threads, a hash set of (refID, found
 // index) pairs, then a block per SM with two full sorts for what they left): 20,000 reads of 1-20 kb
-// on 5,000 references 5.86 -> 1.87 ms, 200,000 reads of 250 bases on references sharing repeats (36
-// copies of a segment) 4.50 -> 2.19 ms, 4,001 reads of 75 bases to 20 kb from host memory 1.28 -> 0.70 ms.
+// on 5,000 references 5.86 -> 1.72 ms, 200,000 reads of 250 bases on references sharing repeats (36
+// copies of a segment) 4.50 -> 2.06 ms, 4,001 reads of 75 bases to 20 kb from host memory 1.28 -> 0.70 ms.
 #pragma once
 #include "mg_lean.cuh"
 
@@ -60,22 +60,22 @@ struct alignas(16) LongSm {
   };
   uint32_t rs[2 * E];  // refID << 11 | seed
   uint32_t ps[2 * E];  // reference position
-  // per share: sorted order (E / 2), kept postings (E / 2), first posting of each seed (NSP); the
-  // seeds' hashes and then the linked references' bitmaps lie over the first two, the candidates'
-  // coverage over the last
-  uint16_t pool[2 * (E + NSP)];
+  // per share: sorted order (E / 2), kept postings (E / 2), first posting and postings of each seed
+  // (NSP each); the seeds with more than a slot's postings and then the linked references' bitmaps lie
+  // over the first two, the candidates' coverage over the last two
+  uint16_t pool[2 * (E + 2 * NSP)];
   uint32_t fm[2 * NW];  // found seeds
   uint16_t fp[2 * NW];  // found seeds before each word of fm
   uint32_t bk[2 * BW];  // starts of diagonal runs
   uint32_t red[2][2][2 * H / 32];
-  uint32_t n_rt[2], over[2], dup[2], n_ends[2], n_out[2], handed;
+  uint32_t ne[2], nx[2], n_rt[2], over[2], dup[2], n_ends[2], n_out[2], handed;
   float hi[2];
   int status[2];
   uint32_t cand_at, ahead;
   Half h[2];
   mg_candidate cb[2][RM];
   uint8_t comp[256];  // complement(upper(byte)), 0 where there is none
-  static_assert(E % 64 == 0 && (E + NSP) % 4 == 0 && NSP % 2 == 0 && 2 * E <= 8192 && NS <= E / 2 && 2 * NS <= 2047 && RT <= 256 && RM < 127, "sizes");
+  static_assert(E % 64 == 0 && E % 4 == 0 && NSP % 2 == 0 && 2 * E <= 8192 && NS <= E / 2 && 2 * NS <= 2047 && RT <= 256 && RM < 127, "sizes");
   static_assert(RM * 8 >= 2 * (RM + 1), "tables over the sums");
 };
 
@@ -83,7 +83,7 @@ struct alignas(16) LongSm {
 // with four blocks per SM, and the plain form's kernel, one block of two warps per read, up to 15 per
 // SM (11,000 reads of 150 bases: 97 us; a block of 256 threads per read with two bitonic sorts per
 // strand, the form before, 1,010 us; room for 256 postings instead of 512 makes no difference).
-using LongSmem = LongSm<128, 2048, 1023, 256, 96>;
+using LongSmem = LongSm<128, 2048, 703, 256, 88>;
 using PlainSmem = LongSm<32, 512, 255, 64, 32>;
 constexpr uint32_t kLgQ = 20480;
 static_assert(4 * (sizeof(LongSmem) + 1024) <= 233472, "four blocks per SM");
@@ -263,9 +263,10 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   const uint32_t k = (uint32_t)ix.k, step = (uint32_t)ix.step;
   uint32_t* rs = S.rs + half * SM::E;
   uint32_t* ps = S.ps + half * SM::E;
-  uint16_t* sx = S.pool + half * (SM::E + SM::NSP);  // sorted order of the kept postings
+  uint16_t* sx = S.pool + half * (SM::E + 2 * SM::NSP);  // sorted order of the kept postings
   uint16_t* kl = sx + kE / 2;                        // the kept postings
-  uint16_t* st = sx + kE;                            // first posting of each seed (kNS + 1)
+  uint16_t* st = sx + kE;                            // first posting of each seed
+  uint16_t* cn = st + (SM::NSP << sh);               // its number of postings
   uint32_t* fm = S.fm + half * SM::NW;
   uint16_t* fp = S.fp + half * SM::NW;
   uint32_t* bk = S.bk + half * SM::BW;
@@ -279,180 +280,154 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   *highest = -1.0f;
   if (L <= k) return kStrandOk;
   const uint32_t ns = (L - k + step - 1) / step;
-  const uint32_t kCovWords = (SM::NSP << sh) / 2;  // over st
+  const uint32_t kCovWords = SM::NSP << sh;  // over st and cn
   if (ns > kNS || (L + 31) / 32 > kCovWords) return kStrandOverflow;
 #pragma unroll 1
   for (uint32_t i = tid; i < kRT; i += G) T.rt[i] = kLgEmpty;
   if (tid == 0) {
     S.n_rt[half] = 0;
     S.over[half] = 0;
+    S.ne[half] = 0;
+    S.nx[half] = 0;
   }
-  // 1. seeds, probe, postings in seed order: every seed's hash first, its slot (or directory entry)
-  //    asked for as it is known; then the bucket sizes, so that the DRAM latency is paid once for all
-  //    seeds and not once per G of them; their prefix sum; then the postings, from L2
-  uint32_t* hb = reinterpret_cast<uint32_t*>(sx);  // the seeds' hashes, over the order arrays
+  lg_sync<SM::H>(bar);
+  // 1. seeds, probe, postings. A seed's slot is read once (random DRAM sectors bound this step: with
+  //    a prefetch, a pass over the counts and one over the postings the tier took 1.70 ms for 20,000 reads
+  //    of 1-20 kb, 1.58 ms so), two seeds in flight per thread; a warp takes room for its seeds' postings from
+  //    the group's cursor, so nothing waits for another warp and the postings lie in no order.
+  uint16_t* xl = kl;                              // seeds with more than a slot's postings (at most kE / 8)
+  uint32_t* xo = reinterpret_cast<uint32_t*>(sx);  // their first posting in the index
+  uint32_t sq2 = 0;                                // this thread's seeds' squared bucket sizes
 #pragma unroll 1
-  for (uint32_t j = tid; j < ns; j += G) {
-    const uint32_t p = j * step;
-    uint32_t h;
-    if (acgt && ix.hlen == 17) {
-      h = hash17_acgt(raw + (strand ? L - 17 - p : p), strand);
-    } else {
-      h = 2166136261u;
-#pragma unroll 1
-      for (int t = 0; t < ix.hlen; t++) {
-        const uint8_t c = strand ? S.comp[raw[L - 1 - p - t]] : upper_dev(raw[p + t]);
-        h = (h * 16777619u) ^ c;
-      }
-      h = ((h >> 28) ^ h) & 0x0FFFFFFFu;
-    }
-    hb[j] = h;
-    if (ix.slots)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(ix.slots + (size_t)h * kSlotVecs));
-    else
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(ix.dir + h));
-  }
-  const uint32_t t0 = ix.slots ? (uint32_t)kSlotPosts : 0u;  // postings of a seed from its slot
-  uint32_t sq2 = 0;   // this thread's seeds' squared bucket sizes
-  bool more = false;  // postings past a slot's
-#pragma unroll 1
-  for (uint32_t j0 = 0; j0 < ns; j0 += 4 * G) {
-    uint32_t c[4];
-    bool found[4];
+  for (uint32_t j0 = 0; j0 < ns; j0 += 2 * G) {
+    uint4 v0[2], v1[2];
+    uint32_t cnt[2], o0[2], hash[2];
 #pragma unroll
-    for (int u = 0; u < 4; u++) {  // four loads in flight
-      const uint32_t j = j0 + u * G + tid;
-      c[u] = 0;
-      found[u] = false;
+    for (int u = 0; u < 2; u++) {
+      const uint32_t j = j0 + u * G + tid, p = j * step;
+      v0[u] = v1[u] = make_uint4(0u, 0u, 0u, 0u);
+      cnt[u] = o0[u] = 0;
+      hash[u] = kLgEmpty;
       if (j < ns) {
-        const uint32_t h = hb[j];  // this thread's own
-        c[u] = ix.slots ? __ldg(reinterpret_cast<const uint32_t*>(ix.slots + (size_t)h * kSlotVecs))
-                        : __ldg(ix.dir + h + 1) - __ldg(ix.dir + h);
-        found[u] = h == ix.empty_hash;
+        uint32_t h;
+        if (acgt && ix.hlen == 17) {
+          h = hash17_acgt(raw + (strand ? L - 17 - p : p), strand);
+        } else {
+          h = 2166136261u;
+#pragma unroll 1
+          for (int t = 0; t < ix.hlen; t++) {
+            const uint8_t c = strand ? S.comp[raw[L - 1 - p - t]] : upper_dev(raw[p + t]);
+            h = (h * 16777619u) ^ c;
+          }
+          h = ((h >> 28) ^ h) & 0x0FFFFFFFu;
+        }
+        hash[u] = h;
+        if (ix.slots) {
+          const uint4* sl = ix.slots + (size_t)h * kSlotVecs;
+          v0[u] = __ldg(sl);
+          v1[u] = __ldg(sl + 1);
+        } else {
+          o0[u] = __ldg(ix.dir + h);
+          cnt[u] = __ldg(ix.dir + h + 1) - o0[u];
+        }
       }
     }
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const uint32_t j = j0 + u * G + tid;
-      if (j0 + u * G >= ns) break;  // group-uniform
-      const uint32_t fb = __ballot_sync(FULL, found[u] || c[u] > 0);
-      more |= c[u] > t0;
-      const uint32_t cnt = min(c[u], kE + 1);
-      sq2 += cnt * cnt;
-      if (j < ns) st[j] = (uint16_t)cnt;
-      if (lane == 0 && (j >> 5) < kNW) fm[j >> 5] = fb;
-    }
-  }
-  lg_sync<SM::H>(bar);
-  uint32_t ne = 0;
-  {
-    const uint32_t C = (ns + G - 1) / G, lo = min(tid * C, ns), hi = min(lo + C, ns);  // consecutive seeds
-    uint32_t own = 0;
 #pragma unroll 1
-    for (uint32_t j = lo; j < hi; j++) own += st[j];  // at most 2 NS (kE + 1) over all seeds: fits 32 bits
-    uint32_t x = own;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(FULL, x, o);
-      if (lane >= (uint32_t)o) x += y;
-    }
-    for (int o = 16; o; o >>= 1) sq2 += min(__shfl_xor_sync(FULL, sq2, o), kLgWork);  // far below 2^32
-    more = __any_sync(FULL, more);
-    if (lane == 31) {
-      red[0][warp] = x;
-      red[1][warp] = min(sq2, kLgWork + 1) | (more ? 0x80000000u : 0u);
-    }
-    if (warp == kW - 1) {  // found seeds before each word: at most 64 words, two a lane
-      const uint32_t nw = (ns + 31) >> 5;
-      const uint32_t c0 = 2 * lane < nw ? __popc(fm[2 * lane]) : 0u,
-                     c1 = 2 * lane + 1 < nw ? __popc(fm[2 * lane + 1]) : 0u;
-      uint32_t f = c0 + c1;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(FULL, f, o);
-        if (lane >= (uint32_t)o) f += y;
+    for (int u = 0; u < 2; u++) {
+      const uint32_t jw = j0 + u * G + warp * 32;  // the warp's first seed
+      if (jw >= ns) break;                         // warp-uniform
+      const uint32_t j = jw + lane, h = u ? hash[1] : hash[0];
+      const uint4 a = u ? v0[1] : v0[0], b = u ? v1[1] : v1[0];
+      uint4 c = make_uint4(0u, 0u, 0u, 0u), d = c;
+      const uint32_t full = ix.slots ? a.x : u ? cnt[1] : cnt[0], o = ix.slots ? a.y : u ? o0[1] : o0[0];
+      if (ix.slots && full > 3) {
+        const uint4* sl = ix.slots + (size_t)h * kSlotVecs;
+        c = __ldg(sl + 2);
+        d = __ldg(sl + 3);
       }
-      if (2 * lane < nw) fp[2 * lane] = (uint16_t)(f - c0 - c1);
-      if (2 * lane + 1 < nw) fp[2 * lane + 1] = (uint16_t)(f - c1);
-    }
-    lg_sync<SM::H>(bar);
-    uint32_t at = x - own, work = 0, any = 0;
-#pragma unroll 1
-    for (uint32_t w = 0; w < kW; w++) {
-      at += w < warp ? red[0][w] : 0u;
-      ne += red[0][w];
-      work += red[1][w] & 0x7FFFFFFFu;
-      any |= red[1][w];
-    }
-    if (ne > kE || work > kLgWork) return kStrandOverflow;  // group-uniform
-    if (ne == 0) return kStrandOk;  // nothing found: the reference skips the strand
-#pragma unroll 1
-    for (uint32_t j = lo; j < hi; j++) {
-      const uint32_t c = st[j];
-      st[j] = (uint16_t)at;
-      at += c;
-    }
-    if (tid == 0) st[ns] = (uint16_t)ne;
-    more = any >> 31;
-  }
-  lg_sync<SM::H>(bar);
-  if (ix.slots)
-#pragma unroll 1
-    for (uint32_t j = tid; j < ns; j += G) {
-      const uint32_t e = st[j], cnt = st[j + 1] - e;
-      if (!cnt) continue;
-      const uint4* sl = ix.slots + (size_t)hb[j] * kSlotVecs;
-      const uint4 v0 = __ldg(sl), v1 = __ldg(sl + 1);
-      uint4 v2 = make_uint4(0u, 0u, 0u, 0u), v3 = v2;
-      if (cnt > 3) {
-        v2 = __ldg(sl + 2);
-        v3 = __ldg(sl + 3);
+      const uint32_t fb = __ballot_sync(FULL, full > 0 || h == ix.empty_hash);
+      const uint32_t n = min(full, kE + 1);
+      sq2 += n * n;
+      uint32_t x = n;
+      for (int t = 1; t < 32; t <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, x, t);
+        if (lane >= (uint32_t)t) x += y;
+      }
+      const uint32_t tot = __shfl_sync(FULL, x, 31);
+      uint32_t base = 0;
+      if (lane == 0) {
+        fm[jw >> 5] = fb;
+        base = atomicAdd(&S.ne[half], tot);  // at most kNS (kE + 1) over a strand: fits 32 bits
+      }
+      base = __shfl_sync(FULL, base, 0);
+      if (base + tot > kE) continue;  // warp-uniform; the strand overflows, seen below
+      const uint32_t e = base + x - n;
+      if (j < ns) {
+        st[j] = (uint16_t)e;
+        cn[j] = (uint16_t)n;
       }
       auto put = [&](uint32_t t, uint32_t ref, uint32_t pos) {
-        if (t < cnt) {
+        if (t < n) {
           rs[e + t] = (ref << 11) | j;
           ps[e + t] = pos;
         }
       };
-      put(0, v0.z, v0.w);
-      put(1, v1.x, v1.y);
-      put(2, v1.z, v1.w);
-      put(3, v2.x, v2.y);
-      put(4, v2.z, v2.w);
-      put(5, v3.x, v3.y);
-      put(6, v3.z, v3.w);
-    }
-  if (more) {  // group-uniform: those past the slots, spread over the threads by posting
+      if (ix.slots) {
+        put(0, a.z, a.w);
+        put(1, b.x, b.y);
+        put(2, b.z, b.w);
+        put(3, c.x, c.y);
+        put(4, c.z, c.w);
+        put(5, d.x, d.y);
+        put(6, d.z, d.w);
+      } else {
 #pragma unroll 1
-    for (uint32_t p0 = tid; p0 < ne; p0 += 4 * G) {
-      uint32_t sj[4];
-      uint2 v[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {  // up to four loads in flight
-        const uint32_t p = p0 + u * G;
-        sj[u] = kLgEmpty;
-        if (p < ne) {
-          uint32_t lo = 0, hi = ns - 1;  // the last seed that starts at or before p
-#pragma unroll 1
-          while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (st[mid] <= p) lo = mid;
-            else hi = mid - 1;
-          }
-          const uint32_t t = p - st[lo];
-          if (t >= t0) {
-            sj[u] = lo;
-            const uint32_t h = hb[lo];
-            const uint32_t o0 =
-                ix.slots ? __ldg(reinterpret_cast<const uint32_t*>(ix.slots + (size_t)h * kSlotVecs) + 1) : __ldg(ix.dir + h);
-            v[u] = __ldg(ix.post + o0 + t);
-          }
+        for (uint32_t t = 0; t < (uint32_t)kSlotPosts && t < n; t++) {
+          const uint2 v = __ldg(ix.post + o + t);
+          put(t, v.x, v.y);
         }
       }
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (sj[u] != kLgEmpty) {
-          rs[p0 + u * G] = (v[u].x << 11) | sj[u];
-          ps[p0 + u * G] = v[u].y;
-        }
+      if (n > (uint32_t)kSlotPosts) {  // at most kE / 8 seeds of the strand
+        const uint32_t i = atomicAdd(&S.nx[half], 1u);
+        xl[i] = (uint16_t)j;
+        xo[i] = o;
+      }
+    }
+  }
+  for (int o = 16; o; o >>= 1) sq2 += min(__shfl_xor_sync(FULL, sq2, o), kLgWork);  // far below 2^32
+  if (lane == 0) red[0][warp] = min(sq2, kLgWork + 1);
+  lg_sync<SM::H>(bar);
+  const uint32_t ne = S.ne[half], nx = S.nx[half];
+  {
+    uint32_t work = 0;
+#pragma unroll 1
+    for (uint32_t w = 0; w < kW; w++) work += red[0][w];
+    if (ne > kE || work > kLgWork) return kStrandOverflow;  // group-uniform
+    if (ne == 0) return kStrandOk;  // nothing found: the reference skips the strand
+  }
+  if (warp == kW - 1) {  // found seeds before each word: at most 64 words, two a lane
+    const uint32_t nw = (ns + 31) >> 5;
+    const uint32_t c0 = 2 * lane < nw ? __popc(fm[2 * lane]) : 0u, c1 = 2 * lane + 1 < nw ? __popc(fm[2 * lane + 1]) : 0u;
+    uint32_t f = c0 + c1;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, f, o);
+      if (lane >= (uint32_t)o) f += y;
+    }
+    if (2 * lane < nw) fp[2 * lane] = (uint16_t)(f - c0 - c1);
+    if (2 * lane + 1 < nw) fp[2 * lane + 1] = (uint16_t)(f - c1);
+  }
+  // the postings past the slots', a warp per eight seeds with four lanes on each
+#pragma unroll 1
+  for (uint32_t i0 = 8 * warp; i0 < nx; i0 += 8 * kW) {
+    const uint32_t i = i0 + (lane >> 2);
+    if (i < nx) {
+      const uint32_t j = xl[i], e = st[j], n = cn[j], o = xo[i];
+#pragma unroll 4
+      for (uint32_t t = (uint32_t)kSlotPosts + (lane & 3u); t < n; t += 4) {
+        const uint2 v = __ldg(ix.post + o + t);
+        rs[e + t] = (v.x << 11) | j;
+        ps[e + t] = v.y;
+      }
     }
   }
   lg_sync<SM::H>(bar);
@@ -469,7 +444,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     if (m) {
       const uint32_t pj = w * 32 + 31 - __clz(m);
       a = st[pj];
-      c = st[pj + 1] - a;
+      c = cn[pj];
       t = i - st[j];  // a stray hit in either bucket shifts the copies by one
       t = t < 2 ? 0 : t - 2;
       if (t >= c) t = 0;

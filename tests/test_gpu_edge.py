@@ -565,7 +565,7 @@ def test_read_beyond_the_oversize_limit_is_refused(golden):
 @pytest.mark.parametrize("slots", [False, True])
 def test_long_read_tier_at_its_edges(tmp_path, slots):
     """The long-read tier at its limits: the shortest read it gets (321 bases), the last and first
-    lengths of its half-blocks (1,023 and 1,024 seeds: 15,376 and 15,377 bases), its longest read
+    lengths of its half-blocks (703 and 704 seeds: 10,576 and 10,577 bases), its longest read
     (20,480) and one past it; on references with a copy, with a segment twice in one reference (two
     postings of a reference under a seed), and with stray seeds of the matched reference elsewhere
     (postings out of seed order); forward, reversed, lowercase and with IUPAC letters; chimeras. With
@@ -591,7 +591,7 @@ def test_long_read_tier_at_its_edges(tmp_path, slots):
     gix, oix = M.Index(image), O.Index(str(path))
     gix.set_probe_slots(slots)
     seqs = []
-    for n in (321, 322, 350, 1100, 6000, 15376, 15377, 20479, 20480, 20481):
+    for n in (321, 322, 350, 1100, 6000, 10576, 10577, 20479, 20480, 20481):
         for src in (core, twice, stray):
             r = src[1000:1000 + n].copy()
             hit = rng.random(n) < 0.02

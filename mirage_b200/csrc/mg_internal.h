@@ -112,6 +112,7 @@ struct Counters {
   bool reran = false;       // the batch ran again with a larger staging arena or oversize workspace
   uint32_t huge_need[4] = {0, 0, 0, 0};  // oversize reads that did not fit: most bases, seeds,
                                          // postings per strand; how many
+  uint32_t n_huge = 0;      // reads that went to the oversize tier
 };
 int read_counters(Workspace& ws, cudaStream_t st, Counters* c);
 // Waits for a launched pipeline and, when the staging arena or the oversize tier's workspace was
@@ -142,6 +143,7 @@ struct mg_index {
   bool chunk_made = false;
   std::mutex mu;
   std::atomic<int> n_servers{0};  // mg_server objects attached to this index
+  std::atomic<int> last_first_tier{1};  // of the last batch run (mg_last_tier_counts)
   mg_tuning tune{};               // launch shapes (mg_set_tuning); zero fields: defaults
   // 2-bit packing of the uploaded bases (mg_classify): host threads and pinned staging
   mg::PackPool* pack_pool = nullptr;

@@ -65,10 +65,12 @@ constexpr int kB3Blocks = 32;
 // or 65,536 postings per strand), one block per read over a workspace sized on demand for the
 // largest such read, 32-bit fields throughout. Hard limits: a read of at most 2,000,000 bases
 // (the relative score's logarithm stays inside its patched domain up to there) and 2^24
-// postings per strand; at most 4 workspaces and 1 GiB.
-constexpr int kHugeThreads = 512;
+// postings per strand; at most 64 workspaces and 1 GiB. A read's time is its strands' sorts, in
+// proportion to the block's threads, and the blocks run side by side: 12 reads of 66-250 kb take
+// 0.88 ms with a workspace each and 1,024 threads (1.13 ms with 512), 3.03 ms with four workspaces and 512 threads.
+constexpr int kHugeThreads = 1024;
 constexpr uint32_t kHugeMaxQ = 2000000, kHugeMaxE = 1u << 24;
-constexpr int kHugeMaxSlabs = 4;
+constexpr int kHugeMaxSlabs = 64;
 constexpr size_t kHugeMaxBytes = size_t(1) << 30;
 
 struct WsLayout {
@@ -120,9 +122,24 @@ struct StageDev {
   unsigned long long* arena_n;
 };
 
+// A read that a dual-strand tier does not take, by one lane: to the next tier's list, or, past all of
+// them with more than kLeanQ bases, to the long-read tier's (n_direct counts those).
+__device__ __forceinline__ void hand_on(const BatchDev& b, uint32_t r, uint32_t* list, unsigned* list_n,
+                                        unsigned* n_direct) {
+  if (b.offs[r + 1] - b.offs[r] > (uint64_t)kLeanQ) {
+    list = b.ovf0b;
+    list_n = b.n_ovf0b;
+    atomicAdd(n_direct, 1u);
+  }
+  list[atomicAdd(list_n, 1u)] = r;
+  b.reads[r] = mg_read_result{};  // not kReadUnscored: a later tier writes this read
+}
+
 // Dual-strand warp tier: every read of the batch, one warp per read (a half-warp per strand),
-// work stealing in chunks of kW1Chunk reads; reads that do not fit go to the 128-posting tier.
-__global__ void __launch_bounds__(kW1Warps * 32, 5) k_classify_dual(DevIndex ix, BatchDev b, StageDev sd, uint32_t chunk) {
+// work stealing in chunks of kW1Chunk reads; reads that do not fit go to the 128-posting tier, reads
+// of more than kLeanQ bases straight to the long-read tier.
+__global__ void __launch_bounds__(kW1Warps * 32, 5) k_classify_dual(DevIndex ix, BatchDev b, StageDev sd, uint32_t chunk,
+                                                                       unsigned* n_direct) {
   __shared__ DualSmem sm[kW1Warps];
   __shared__ uint8_t comp[256];
   for (int c = threadIdx.x; c < 256; c += blockDim.x) comp[c] = complement_dev(upper_dev((uint8_t)c));
@@ -138,11 +155,7 @@ __global__ void __launch_bounds__(kW1Warps * 32, 5) k_classify_dual(DevIndex ix,
     const uint32_t end = (uint32_t)(end64 < b.n ? end64 : b.n);
     for (uint32_t r = base; r < end; r++) {
       if (!process_read_dual(ix, b, r, S, comp, sd.stage, sd.arena, sd.arena_cap, sd.arena_n, b.err)) {
-        if (lane == 0) {
-          unsigned at = atomicAdd(b.n_ovf0, 1u);
-          b.ovf0[at] = r;
-          b.reads[r] = mg_read_result{};  // not kReadUnscored: a later tier writes this read
-        }
+        if (lane == 0) hand_on(b, r, b.ovf0, b.n_ovf0, n_direct);
       }
       __syncwarp();
     }
@@ -298,7 +311,8 @@ template <int Cap, int Warps>
 __global__ void __launch_bounds__(Warps * 32) k_classify_dual_list(DevIndex ix, BatchDev b, StageDev sd,
                                                                      const uint32_t* list, const unsigned* list_n,
                                                                      unsigned* cursor, uint32_t* next,
-                                                                     unsigned* next_n, int all_reads) {
+                                                                     unsigned* next_n, int all_reads,
+                                                                     unsigned* n_direct) {
   __shared__ DualSmemT<Cap> sm[Warps];
   __shared__ uint8_t comp[256];
   for (int c = threadIdx.x; c < 256; c += blockDim.x) comp[c] = complement_dev(upper_dev((uint8_t)c));
@@ -313,11 +327,7 @@ __global__ void __launch_bounds__(Warps * 32) k_classify_dual_list(DevIndex ix, 
     if (item >= n) break;
     const uint32_t r = all_reads ? item : list[item];
     if (!process_read_dual(ix, b, r, S, comp, sd.stage, sd.arena, sd.arena_cap, sd.arena_n, b.err)) {
-      if (lane == 0) {
-        unsigned at = atomicAdd(next_n, 1u);
-        next[at] = r;
-        b.reads[r] = mg_read_result{};  // not kReadUnscored: a later tier writes this read
-      }
+      if (lane == 0) hand_on(b, r, next, next_n, n_direct);
     }
     __syncwarp();
   }
@@ -501,33 +511,36 @@ __global__ void k_unpack_exceptions(const uint64_t* exc, uint64_t n_exc, uint64_
 // contiguous array in read order.
 constexpr int kScanBlock = 1024;
 
-__global__ void k_count_sums(const mg_read_result* reads, uint64_t n, unsigned long long* block_sums) {
+// Block sums of the counts, and, by the last block to finish, their exclusive scan (one launch for
+// both). chain (optional): candidates of earlier chunks of the same batch; the scan starts there and
+// leaves the new running total behind, so chunk offsets are offsets into the batch's output.
+__global__ void __launch_bounds__(kScanBlock) k_count_scan(const mg_read_result* reads, uint64_t n,
+                                                           unsigned long long* block_sums, unsigned* done,
+                                                           unsigned long long* total, unsigned long long* chain) {
   __shared__ unsigned long long s[kScanBlock / 32];
-  uint64_t i = (uint64_t)blockIdx.x * kScanBlock + threadIdx.x;
-  unsigned long long v = i < n ? (unsigned long long)(reads[i].n_fwd + reads[i].n_rc) : 0ull;
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint64_t nb = gridDim.x, r = (uint64_t)blockIdx.x * kScanBlock + threadIdx.x;
+  unsigned long long v = r < n ? (unsigned long long)(reads[r].n_fwd + reads[r].n_rc) : 0ull;
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+  if (lane == 0) s[wid] = v;
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long t = 0;
     for (int w = 0; w < kScanBlock / 32; w++) t += s[w];
     block_sums[blockIdx.x] = t;
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
   }
-}
-
-// Exclusive scan of the per-block candidate counts, one block of kScanBlock threads in tiles.
-// chain (optional): candidates of earlier chunks of the same batch; the scan starts there and
-// leaves the new running total behind, so chunk offsets are offsets into the batch's output.
-__global__ void __launch_bounds__(kScanBlock) k_scan_sums(unsigned long long* block_sums, uint64_t nb,
-                                                          unsigned long long* total, unsigned long long* chain) {
-  __shared__ unsigned long long s[kScanBlock / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
   const unsigned long long base = chain ? *chain : 0ull;
   unsigned long long carry = base;
   for (uint64_t t0 = 0; t0 < nb; t0 += kScanBlock) {
     const uint64_t i = t0 + threadIdx.x;
-    const unsigned long long v = i < nb ? block_sums[i] : 0ull;
-    unsigned long long x = v;
+    const unsigned long long c = i < nb ? __ldcg(block_sums + i) : 0ull;
+    unsigned long long x = c;
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
@@ -539,7 +552,7 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_sums(unsigned long long* bl
       wb += w < wid ? s[w] : 0ull;
       tile += s[w];
     }
-    if (i < nb) block_sums[i] = carry + wb + x - v;
+    if (i < nb) block_sums[i] = carry + wb + x - c;
     carry += tile;
     __syncthreads();
   }
@@ -547,6 +560,21 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_sums(unsigned long long* bl
     *total = carry - base;
     if (chain) *chain = carry;
   }
+}
+
+// One read's candidates to their place in the output.
+__device__ __forceinline__ void scatter_read(mg_read_result* reads, uint64_t i, unsigned long long off, const StageDev& sd,
+                                             mg_candidate* out, uint64_t cap, int* err) {
+  mg_read_result rr = reads[i];
+  const uint32_t tot = rr.n_fwd + rr.n_rc;
+  const mg_candidate* src = tot > (uint32_t)kSlots ? sd.arena + rr.cand_off : sd.stage + i * kSlots;
+  if (off + tot > cap) {
+    atomicOr(err, kErrOutput);
+  } else {
+    for (uint32_t c = 0; c < tot; c++) out[off + c] = src[c];
+  }
+  rr.cand_off = (uint32_t)off;
+  reads[i] = rr;
 }
 
 __global__ void k_scatter(mg_read_result* reads, uint64_t n, const unsigned long long* block_sums, StageDev sd,
@@ -564,18 +592,37 @@ __global__ void k_scatter(mg_read_result* reads, uint64_t n, const unsigned long
   __syncthreads();
   unsigned long long wb = 0;
   for (int w = 0; w < wid; w++) wb += s[w];
-  if (i >= n) return;
-  const unsigned long long off = block_sums[blockIdx.x] + wb + x - v;
-  mg_read_result rr = reads[i];
-  const uint32_t tot = rr.n_fwd + rr.n_rc;
-  const mg_candidate* src = tot > (uint32_t)kSlots ? sd.arena + rr.cand_off : sd.stage + i * kSlots;
-  if (off + tot > cap) {
-    atomicOr(err, kErrOutput);
-  } else {
-    for (uint32_t c = 0; c < tot; c++) out[off + c] = src[c];
+  if (i < n) scatter_read(reads, i, block_sums[blockIdx.x] + wb + x - v, sd, out, cap, err);
+}
+
+// The whole compaction of a batch of up to kScanSmall reads, one block: a launch instead of two, which
+// is what such a batch waits for.
+constexpr uint64_t kScanSmall = 2 * kScanBlock;
+__global__ void __launch_bounds__(kScanBlock) k_compact_small(mg_read_result* reads, uint64_t n, unsigned long long* total,
+                                                              StageDev sd, mg_candidate* out, uint64_t cap, int* err) {
+  __shared__ unsigned long long s[kScanBlock / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned long long carry = 0;
+  for (uint64_t t0 = 0; t0 < n; t0 += kScanBlock) {
+    const uint64_t i = t0 + threadIdx.x;
+    const unsigned long long v = i < n ? (unsigned long long)(reads[i].n_fwd + reads[i].n_rc) : 0ull;
+    unsigned long long x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) s[wid] = x;
+    __syncthreads();
+    unsigned long long wb = 0, tile = 0;
+    for (int w = 0; w < kScanBlock / 32; w++) {
+      wb += w < wid ? s[w] : 0ull;
+      tile += s[w];
+    }
+    if (i < n) scatter_read(reads, i, carry + wb + x - v, sd, out, cap, err);
+    carry += tile;
+    __syncthreads();
   }
-  rr.cand_off = (uint32_t)off;
-  reads[i] = rr;
+  if (threadIdx.x == 0) *total = carry;
 }
 
 // Index construction: directory from the ascending TOC (dir[h] = first posting of the first
@@ -1131,7 +1178,9 @@ int ensure_workspace(Workspace& w, uint64_t n_reads, uint64_t n_bases, bool host
 // Counters in w_ctr (device): 0 n_cands(u64) | 8 arena_n(u64) | 16 err | 20 work | 28 work2 |
 // 32 n_ovf2 | 36 work3 | 40 total(u64) | 48 n_ovf0 | 56 n_ovf0b | 60 work0b | 64 n_large |
 // 68 work of the long-read tier | 72 n_ovf0c | 76 work0c | 80 n_small | 88 n_ovf3 (the global tier's
-// leftovers) | 92 work4 | 96 oversize need: most bases, seeds, postings, reads waiting (4 x u32)
+// leftovers) | 92 work4 | 96 oversize need: most bases, seeds, postings, reads waiting (4 x u32) |
+// reads too long for the dual-strand tiers that the first one met: 24 (64 postings), 112 (128), 116 (256) |
+// 120 blocks done in k_count_scan
 int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs, const uint8_t* d_bases,
                         mg_read_result* d_reads, mg_candidate* d_out, uint64_t cap, cudaStream_t st,
                         bool plain, unsigned long long* chain, const ChainSync* cs) {
@@ -1222,14 +1271,27 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
         CU(cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming));
         CU(cudaEventCreateWithFlags(&w.join, cudaEventDisableTiming));
       }
-      if (sh.first_tier == 1)
-        k_classify_dual<<<sh.dual_blocks_per_sm * sms, kW1Warps * 32, 0, st>>>(ix->dix, b, sd, sh.steal_chunk);
-      // tiers of 64, 128 and 256 postings per strand, each over the one before's leftovers
-      if (sh.first_tier <= 2)
+      // tiers of 64, 128 and 256 postings per strand, each over the one before's leftovers. The last
+      // runs only for indexes whose reads start beyond the first (their strands' random hits fill the
+      // smaller ones); elsewhere a strand of more than 128 postings lies in repeats, and the long-read
+      // tier takes it (200,000 reads of 250 bases, 16,000 such: @@)
+      // a small batch is spread over the warps, a read each if it can be (a chunk per warp waits for its
+      // reads in turn: 16 reads 20 us in four chunks, 6 us so)
+      const unsigned dual_warps = sh.dual_blocks_per_sm * sms * kW1Warps;
+      const unsigned chunk = std::min(sh.steal_chunk, (unsigned)std::max<uint64_t>(1, (n + dual_warps - 1) / dual_warps));
+      ix->last_first_tier = (int)sh.first_tier;
+      if (sh.first_tier == 1) {
+        k_classify_dual<<<(unsigned)std::min<uint64_t>(sh.dual_blocks_per_sm * sms, (n + kW1Warps * chunk - 1) / (kW1Warps * chunk)),
+                          kW1Warps * 32, 0, st>>>(ix->dix, b, sd, chunk, (unsigned*)(ctr + 24));
         k_classify_dual_list<128, kW2Warps><<<sh.second_blocks_per_sm * sms, kW2Warps * 32, 0, st>>>(
-            ix->dix, b, sd, b.ovf0, b.n_ovf0, b.work0b, ovf0c, n_ovf0c, sh.first_tier == 2);
-      k_classify_dual_list<256, kW3Warps><<<sh.third_blocks_per_sm * sms, kW3Warps * 32, 0, st>>>(
-          ix->dix, b, sd, ovf0c, n_ovf0c, work0c, b.ovf0b, b.n_ovf0b, sh.first_tier == 3);
+            ix->dix, b, sd, b.ovf0, b.n_ovf0, b.work0b, b.ovf0b, b.n_ovf0b, 0, (unsigned*)(ctr + 24));
+      } else {
+        if (sh.first_tier == 2)
+          k_classify_dual_list<128, kW2Warps><<<sh.second_blocks_per_sm * sms, kW2Warps * 32, 0, st>>>(
+              ix->dix, b, sd, b.ovf0, b.n_ovf0, b.work0b, ovf0c, n_ovf0c, 1, (unsigned*)(ctr + 112));
+        k_classify_dual_list<256, kW3Warps><<<sh.third_blocks_per_sm * sms, kW3Warps * 32, 0, st>>>(
+            ix->dix, b, sd, ovf0c, n_ovf0c, work0c, b.ovf0b, b.n_ovf0b, sh.first_tier == 3, (unsigned*)(ctr + 116));
+      }
       // the reads the dual tiers handed on go through the other tiers on the side stream, beside
       // the dual tier's finishing pass (different reads, disjoint slots; arena space by atomics)
       CU(cudaEventRecord(w.fork, st));
@@ -1245,14 +1307,18 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
     }
     CU(cudaGetLastError());
     if (tm) CU(cudaEventRecord(ix->ev[6], st));
-    const uint64_t nb = (n + kScanBlock - 1) / kScanBlock;
     unsigned long long* sums = w.sums.as<unsigned long long>();
-    k_count_sums<<<(unsigned)nb, kScanBlock, 0, st>>>(d_reads, n, sums);
-    if (cs && cs->wait_prev) CU(cudaStreamWaitEvent(st, cs->wait_prev, 0));
-    k_scan_sums<<<1, kScanBlock, 0, st>>>(sums, nb, (unsigned long long*)(ctr + 40), chain);
-    if (cs && cs->snap) CU(cudaMemcpyAsync(cs->snap, chain, 8, cudaMemcpyDeviceToHost, st));
-    if (cs && cs->scanned) CU(cudaEventRecord(cs->scanned, st));
-    k_scatter<<<(unsigned)nb, kScanBlock, 0, st>>>(d_reads, n, sums, sd, d_out, cap, b.err);
+    if (n <= kScanSmall && !chain) {
+      k_compact_small<<<1, kScanBlock, 0, st>>>(d_reads, n, (unsigned long long*)(ctr + 40), sd, d_out, cap, b.err);
+    } else {
+      const uint64_t nb = (n + kScanBlock - 1) / kScanBlock;
+      if (cs && cs->wait_prev) CU(cudaStreamWaitEvent(st, cs->wait_prev, 0));
+      k_count_scan<<<(unsigned)nb, kScanBlock, 0, st>>>(d_reads, n, sums, (unsigned*)(ctr + 120),
+                                                        (unsigned long long*)(ctr + 40), chain);
+      if (cs && cs->snap) CU(cudaMemcpyAsync(cs->snap, chain, 8, cudaMemcpyDeviceToHost, st));
+      if (cs && cs->scanned) CU(cudaEventRecord(cs->scanned, st));
+      k_scatter<<<(unsigned)nb, kScanBlock, 0, st>>>(d_reads, n, sums, sd, d_out, cap, b.err);
+    }
     if (tm) CU(cudaEventRecord(ix->ev[7], st));
     CU(cudaGetLastError());
   }
@@ -1268,6 +1334,7 @@ int read_counters(Workspace& w, cudaStream_t st, Counters* c) {
   std::memcpy(&need, h + 8, 8);
   std::memcpy(&total, h + 40, 8);
   std::memcpy(c->huge_need, h + 96, 16);
+  std::memcpy(&c->n_huge, h + 88, 4);
   c->n_cands = total;
   c->arena_need = need;
   return MG_OK;
@@ -1317,6 +1384,13 @@ int complete_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_
     rc = run_pipeline(ix, w, n, d_offs, d_bases, d_reads, d_out, cap, st, plain);
     c->reran = true;
     if (rc == MG_OK) rc = read_counters(w, st, c);
+  }
+  // more oversize reads than workspaces: the next such batch gets one per read (if there is no memory
+  // for that, the tier sizes its workspace anew when a batch needs it)
+  if (rc == MG_OK && w.hslabs && (int)std::min<uint32_t>(c->n_huge, kHugeMaxSlabs) > w.hslabs) {
+    Counters more;
+    more.huge_need[3] = c->n_huge;
+    grow_oversize(ix, w, more);
   }
   return rc;
 }
@@ -1801,11 +1875,22 @@ int mg_last_tier_counts(mg_index* ix, uint32_t* counts7) {
   uint8_t h[128];
   CU(cudaStreamSynchronize(ix->stream));
   CU(cudaMemcpy(h, ix->ws.ctr.p, sizeof(h), cudaMemcpyDeviceToHost));
-  // the lists' counters (run_pipeline): left by the 64-, 128- and 256-posting dual tiers (the last
-  // also as the general warp tier's entry, which has no tier of its own any more), by the long-read
-  // tier's half-blocks and its whole block, and in all for the global-memory tier
-  static const int at[7] = {48, 72, 56, 56, 80, 64, 32};
-  for (int i = 0; i < 7; i++) std::memcpy(&counts7[i], h + at[i], 4);
+  // the lists' counters (run_pipeline): left by the 64-, 128- and 256-posting dual tiers (with the reads
+  // too long for them, which skip the rest; the tiers not run count what passes them; the last also as
+  // the general warp tier's entry, which has no tier of its own any more), by the long-read tier's
+  // half-blocks and its whole block, and in all for the global-memory tier
+  auto u32 = [&](int o) {
+    uint32_t v;
+    std::memcpy(&v, h + o, 4);
+    return v;
+  };
+  const int first = ix->last_first_tier;
+  counts7[0] = first == 1 ? u32(48) + u32(24) : 0;
+  counts7[1] = first == 1 ? u32(56) : first == 2 ? u32(72) + u32(112) : 0;
+  counts7[2] = counts7[3] = u32(56);
+  counts7[4] = u32(80);
+  counts7[5] = u32(64);
+  counts7[6] = u32(32);
   return MG_OK;
 }
 

@@ -174,8 +174,8 @@ __device__ __forceinline__ uint32_t walk_record(const DevIndex& ix, const uint8_
                   (jj >> 8) * step + step, k);
 }
 
-// Finishing pass of the dual-strand tiers over the reads they left kReadUnscored, a warp per 32
-// consecutive reads. A read's run records (forward strand first, each strand in ascending refID;
+// Finishing pass of the dual-strand tiers over the reads they left kReadUnscored, a warp per per_warp
+// (up to 32) consecutive reads. A read's run records (forward strand first, each strand in ascending refID;
 // see process_read_dual) name the run ends of the references whose longest run is M. The warp
 // walks its reads' records one per lane (walk_record), so that reads with many records or long
 // walks do not hold the other lanes; then each read's lane groups its records by reference: the
@@ -183,7 +183,8 @@ __device__ __forceinline__ uint32_t walk_record(const DevIndex& ix, const uint8_
 // is a candidate whose Score, percentage and relative score (MatrixCPU.cpp:18-214,
 // MatrixResult.cpp:21-29) replace its records, compacted in place; then the strand merge and top
 // group as write_read_result_s (Analyser.cpp:592-611, 388).
-__global__ void __launch_bounds__(kFinThreads) k_finish_dual(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd) {
+__global__ void __launch_bounds__(kFinThreads) k_finish_dual(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd,
+                                                             uint32_t per_warp) {
   const unsigned FULL = 0xffffffffu;
   __shared__ uint8_t comp[256];
   __shared__ uint32_t covs[kFinThreads * kCovStride];
@@ -194,10 +195,10 @@ __global__ void __launch_bounds__(kFinThreads) k_finish_dual(const __grid_consta
   uint32_t* cov = covs + threadIdx.x * kCovStride;
   uint32_t* zw = walks[threadIdx.x >> 5];
   const uint32_t k = (uint32_t)ix.k, step = (uint32_t)ix.step;
-  // a warp takes 32 consecutive reads, one per lane
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < b.n;
-       base += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t r = base + lane;
+  // a warp takes per_warp consecutive reads, one per lane
+  for (uint64_t base = ((uint64_t)blockIdx.x * (kFinThreads / 32) + (threadIdx.x >> 5)) * per_warp; base < b.n;
+       base += (uint64_t)gridDim.x * (kFinThreads / 32) * per_warp) {
+    const uint64_t r = lane < (int)per_warp ? base + lane : b.n;
     mg_read_result rr{};
     bool mine = false;
     if (r < b.n) {
@@ -1274,7 +1275,7 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
       // tiers of 64, 128 and 256 postings per strand, each over the one before's leftovers. The last
       // runs only for indexes whose reads start beyond the first (their strands' random hits fill the
       // smaller ones); elsewhere a strand of more than 128 postings lies in repeats, and the long-read
-      // tier takes it (200,000 reads of 250 bases, 16,000 such: @@)
+      // tier takes it (200,000 reads of 250 bases, 16,000 such: 2.08 ms with it, 1.97 ms without)
       // a small batch is spread over the warps, a read each if it can be (a chunk per warp waits for its
       // reads in turn: 16 reads 20 us in four chunks, 6 us so)
       const unsigned dual_warps = sh.dual_blocks_per_sm * sms * kW1Warps;
@@ -1299,9 +1300,13 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
       const int rc = further_tiers(w.side);
       if (rc) return rc;
       CU(cudaEventRecord(w.join, w.side));
-      k_finish_dual<<<(unsigned)std::min<uint64_t>((n + kFinThreads - 1) / kFinThreads,
+      // 32 reads to a warp when they fill the GPU; fewer for a batch that leaves warps idle, so that its
+      // walks, a record per lane, take one round each (20,011 reads: 26 us with 32, 18 us with 8;
+      // 1 M reads: 222 us with 32)
+      const uint32_t per_warp = n < 65536 ? 8 : 32, per_block = kFinThreads / 32 * per_warp;
+      k_finish_dual<<<(unsigned)std::min<uint64_t>((n + per_block - 1) / per_block,
                                                    (uint64_t)sms * sh.finish_blocks_per_sm),
-                      kFinThreads, 0, st>>>(ix->dix, b, sd);
+                      kFinThreads, 0, st>>>(ix->dix, b, sd, per_warp);
       if (tm) CU(cudaEventRecord(ix->ev[1], st));
       CU(cudaStreamWaitEvent(st, w.join, 0));
     }

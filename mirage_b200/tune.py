@@ -38,7 +38,7 @@ SHORT_GRID = {
     "third_blocks_per_sm": [2, 4, 6],
     "finish_blocks_per_sm": [2, 4, 8],
 }
-LONG_GRID = {"long_blocks_per_sm": [1, 2]}
+LONG_GRID = {"long_blocks_per_sm": [2, 3, 4]}
 E2E_GRID = {"chunks": [4, 6, 8], "weighted_chunks": [1, 2], "pack_bases": [1, 2]}
 
 

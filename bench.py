@@ -17,7 +17,7 @@ flush is needed between steps.
   served      the served form (mg_server_*): saturated reads/s with requests of log-uniform
               size in [1, 50000] reads, then p50/p99 request latency under Poisson arrivals at
               25/50/75/90% of that rate.
-  roofline    the warp tiers (the dual-strand kernel and the general warp kernel, which take
+  roofline    the warp tiers (the dual-strand kernel and the long-read kernel, which take
               every read once between them; 97% of a step): algorithmic bytes per step / their
               CUDA-event time, against the measured HBM copy bandwidth (peak) and against the
               random 32-byte-sector gather bandwidth measured in the same run (gather_peak).
@@ -45,9 +45,11 @@ sys.path.insert(0, ROOT)
 
 SEED = 2024
 N_READS = 1_000_000
-# kernels one batched call launches: dual-strand tier, second dual-strand tier (its leftovers),
-# third dual-strand tier, the finishing pass, long-read tier, global tier, candidate count, scan, scatter
-LAUNCHES_PER_BATCH = 9
+# kernels one batched call launches: dual-strand tier, second dual-strand tier (its leftovers), the
+# finishing pass, long-read tier, global tier, candidate counts and their scan, scatter (an index whose
+# reads start at the second tier launches the third instead of the first; batches of up to 2,048 reads
+# launch one kernel for the last two)
+LAUNCHES_PER_BATCH = 7
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_classify_dual launch on the
 # default workload (1,000,000 reads, scale 1.0): a constant from one ncu capture of this kernel,
 # not a measurement of this run

@@ -1088,9 +1088,10 @@ static Shapes shapes(const mg_index* ix) {
   s.first_tier = pick(t.first_tier, 1, 1, 3);
   s.dual_blocks_per_sm = pick(t.dual_blocks_per_sm, (unsigned)occ_dual, 1, (unsigned)occ_dual);
   s.steal_chunk = pick(t.steal_chunk, kW1Chunk, 1, 64);
-  // the 128-posting tier takes the first tier's few leftovers (one block per SM), or every read
-  s.second_blocks_per_sm = pick(t.second_blocks_per_sm, s.first_tier == 2 ? (unsigned)occ_second : 1u, 1,
-                                (unsigned)occ_second);
+  // the 128-posting tier at full occupancy also over the first tier's leftovers: an idle block costs next
+  // to nothing, and with one block per SM 19,000 of 200,000 reads on references with repeats waited in
+  // turn (170 us, 74 us so)
+  s.second_blocks_per_sm = pick(t.second_blocks_per_sm, (unsigned)occ_second, 1, (unsigned)occ_second);
   s.third_blocks_per_sm = pick(t.third_blocks_per_sm, (unsigned)occ_third, 1, (unsigned)occ_third);
   s.pack_bases = pick(t.pack_bases, 1, 1, 2);
   s.finish_blocks_per_sm = pick(t.finish_blocks_per_sm, 8, 1, 8);
@@ -1240,18 +1241,22 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
     // ev[3..4] long-read tier, ev[4..5] global tier, ev[6..7] compaction
     if (tm) CU(cudaEventRecord(ix->ev[0], st));
     const Shapes sh = shapes(ix);
+    // no more blocks than the batch has work for, per_block reads to one
+    auto grid = [&](unsigned blocks, unsigned per_block) {
+      return (unsigned)std::min<uint64_t>(blocks, (n + per_block - 1) / per_block);
+    };
     // the tiers behind the dual-strand ones and the plain form's kernel, on stream s
     auto further_tiers = [&](cudaStream_t s) -> int {
       if (tm) CU(cudaEventRecord(ix->ev[2], s));
       if (tm) CU(cudaEventRecord(ix->ev[3], s));
       if (ix->dix.n_refs <= (1u << 21))
-        k_classify_long<<<sh.long_blocks_per_sm * sms, 2 * LongSmem::H, sizeof(LongSmem), s>>>(
+        k_classify_long<<<grid(sh.long_blocks_per_sm * sms, 1), 2 * LongSmem::H, sizeof(LongSmem), s>>>(
             ix->dix, b, sd, b.ovf0b, b.n_ovf0b, work_long, b.ovf2, b.n_ovf2, n_small, n_large);
       else
-        k_classify_block<kB2Threads><<<(unsigned)sms, kB2Threads, l2.total, s>>>(
+        k_classify_block<kB2Threads><<<grid(sms, 1), kB2Threads, l2.total, s>>>(
             ix->dix, b, sd, b.ovf0b, b.n_ovf0b, b.work2, b.ovf2, b.n_ovf2, nullptr, l2, c2, 0);
       if (tm) CU(cudaEventRecord(ix->ev[4], s));
-      k_classify_block<kB3Threads><<<kB3Blocks, kB3Threads, 0, s>>>(ix->dix, b, sd, b.ovf2, b.n_ovf2, b.work3, ovf3,
+      k_classify_block<kB3Threads><<<grid(kB3Blocks, 1), kB3Threads, 0, s>>>(ix->dix, b, sd, b.ovf2, b.n_ovf2, b.work3, ovf3,
                                                                     n_ovf3, w.gws.as<uint8_t>(), l3, c3, !w.hmode);
       // the oversize tier, once a batch of this workspace has needed it: one block while it has
       // no workspace (it only sizes the reads it gets)
@@ -1282,15 +1287,14 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
       const unsigned chunk = std::min(sh.steal_chunk, (unsigned)std::max<uint64_t>(1, (n + dual_warps - 1) / dual_warps));
       ix->last_first_tier = (int)sh.first_tier;
       if (sh.first_tier == 1) {
-        k_classify_dual<<<(unsigned)std::min<uint64_t>(sh.dual_blocks_per_sm * sms, (n + kW1Warps * chunk - 1) / (kW1Warps * chunk)),
-                          kW1Warps * 32, 0, st>>>(ix->dix, b, sd, chunk, (unsigned*)(ctr + 24));
-        k_classify_dual_list<128, kW2Warps><<<sh.second_blocks_per_sm * sms, kW2Warps * 32, 0, st>>>(
+        k_classify_dual<<<grid(sh.dual_blocks_per_sm * sms, kW1Warps * chunk), kW1Warps * 32, 0, st>>>(ix->dix, b, sd, chunk, (unsigned*)(ctr + 24));
+        k_classify_dual_list<128, kW2Warps><<<grid(sh.second_blocks_per_sm * sms, kW2Warps), kW2Warps * 32, 0, st>>>(
             ix->dix, b, sd, b.ovf0, b.n_ovf0, b.work0b, b.ovf0b, b.n_ovf0b, 0, (unsigned*)(ctr + 24));
       } else {
         if (sh.first_tier == 2)
-          k_classify_dual_list<128, kW2Warps><<<sh.second_blocks_per_sm * sms, kW2Warps * 32, 0, st>>>(
+          k_classify_dual_list<128, kW2Warps><<<grid(sh.second_blocks_per_sm * sms, kW2Warps), kW2Warps * 32, 0, st>>>(
               ix->dix, b, sd, b.ovf0, b.n_ovf0, b.work0b, ovf0c, n_ovf0c, 1, (unsigned*)(ctr + 112));
-        k_classify_dual_list<256, kW3Warps><<<sh.third_blocks_per_sm * sms, kW3Warps * 32, 0, st>>>(
+        k_classify_dual_list<256, kW3Warps><<<grid(sh.third_blocks_per_sm * sms, kW3Warps), kW3Warps * 32, 0, st>>>(
             ix->dix, b, sd, ovf0c, n_ovf0c, work0c, b.ovf0b, b.n_ovf0b, sh.first_tier == 3, (unsigned*)(ctr + 116));
       }
       // the reads the dual tiers handed on go through the other tiers on the side stream, beside

@@ -62,6 +62,7 @@ struct Workspace {
   DevBuf hws;
   int hmode = 0;
   int hslabs = 0;
+  bool hshort = false;  // the device had no memory for as many slabs as reads
   uint32_t hq = 0, hseeds = 0, he = 0, hc = 0;
   // the stream on which the tiers after the dual tier run beside its finishing pass, and the
   // events that fork it from and join it back to the call's stream (made at first use)
@@ -72,6 +73,7 @@ struct Workspace {
                       &hws})
       b->release();
     hmode = hslabs = 0;
+    hshort = false;
     hq = hseeds = he = hc = 0;
     if (side) cudaStreamDestroy(side);
     if (fork) cudaEventDestroy(fork);

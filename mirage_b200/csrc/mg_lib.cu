@@ -27,6 +27,7 @@
 #include "mg_lean.cuh"
 #include "mg_dual.cuh"
 #include "mg_long.cuh"
+#include "mg_slabs.h"
 #include "mhm.h"
 
 namespace mg {
@@ -1350,26 +1351,45 @@ int read_counters(Workspace& w, cudaStream_t st, Counters* c) {
 }
 
 // Grow the oversize tier's slabs to hold every read the last run sized (and every read the old
-// slabs held): one slab per waiting read, up to kHugeMaxSlabs and kHugeMaxBytes in all.
+// slabs held): one slab per waiting read, up to kHugeMaxSlabs and kHugeMaxBytes in all, fewer when
+// the device has no memory for them.
 static int grow_oversize(mg_index* ix, Workspace& w, const Counters& c) {
   const uint32_t q = std::max(w.hq, c.huge_need[0]), seeds = std::max(w.hseeds, c.huge_need[1]);
   uint32_t e = 1;
   while (e < std::max(w.he, c.huge_need[2])) e <<= 1;
   const uint32_t cand = std::min<uint32_t>(std::min<uint32_t>(e, std::max<uint32_t>(ix->dix.n_refs, 1)), 65535);
   const WsLayout l = ws_layout((int)q, (int)seeds, (int)e, (int)cand, true);
-  const uint64_t fit = std::max<uint64_t>(1, kHugeMaxBytes / l.total);
-  const int slabs = (int)std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(w.hslabs, c.huge_need[3]), kHugeMaxSlabs), fit);
-  if (w.hws.alloc(l.total * (size_t)slabs)) {
+  const int slabs = take_slabs(slabs_wanted(w.hslabs, c.huge_need[3], kHugeMaxSlabs, l.total, kHugeMaxBytes), 1,
+                               [&](int n) { return w.hws.alloc(l.total * (size_t)n) == 0; });
+  if (!slabs) {
     w.hslabs = 0;
     w.hq = w.hseeds = w.he = w.hc = 0;
     return set_error(MG_ERR_OOM, "oversize-read workspace");
   }
   w.hslabs = slabs;
+  w.hshort = false;
   w.hq = q;
   w.hseeds = seeds;
   w.he = e;
   w.hc = cand;
   return MG_OK;
+}
+
+// After a batch that ran with fewer slabs than it had oversize reads: more slabs of the same size for
+// the next one, beside the old ones until they are there. Where there is no memory for more, the old
+// ones stay, and this workspace does not ask again before its slabs are sized anew.
+static void add_slabs(Workspace& w, uint32_t n_huge) {
+  const WsLayout l = ws_layout((int)w.hq, (int)w.hseeds, (int)w.he, (int)w.hc, true);
+  const int want = slabs_wanted(w.hslabs, n_huge, kHugeMaxSlabs, l.total, kHugeMaxBytes);
+  if (want <= w.hslabs || w.hshort) return;
+  DevBuf more;
+  const int slabs = take_slabs(want, w.hslabs + 1, [&](int n) { return more.alloc(l.total * (size_t)n) == 0; });
+  if (slabs) {
+    std::swap(w.hws, more);
+    more.release();
+    w.hslabs = slabs;
+  }
+  w.hshort = slabs != want;
 }
 
 int complete_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs, const uint8_t* d_bases,
@@ -1394,13 +1414,7 @@ int complete_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_
     c->reran = true;
     if (rc == MG_OK) rc = read_counters(w, st, c);
   }
-  // more oversize reads than workspaces: the next such batch gets one per read (if there is no memory
-  // for that, the tier sizes its workspace anew when a batch needs it)
-  if (rc == MG_OK && w.hslabs && (int)std::min<uint32_t>(c->n_huge, kHugeMaxSlabs) > w.hslabs) {
-    Counters more;
-    more.huge_need[3] = c->n_huge;
-    grow_oversize(ix, w, more);
-  }
+  if (rc == MG_OK && w.hslabs) add_slabs(w, c->n_huge);
   return rc;
 }
 

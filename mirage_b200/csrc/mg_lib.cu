@@ -336,15 +336,17 @@ __global__ void __launch_bounds__(Warps * 32) k_classify_dual_list(DevIndex ix, 
 }
 
 // Long-read tier over the dual tiers' leftovers and the plain form's, a block per read with work
-// stealing (the next read is taken while this one is classified); its own leftovers go to the
+// stealing (the next read is taken while this one is classified), in two classes: LongSmem, then RestSmem
+// over what that leaves (its launch costs a batch without such reads 2.5 us), whose own leftovers go to the
 // global-memory tier.
-__global__ void __launch_bounds__(2 * LongSmem::H, 4) k_classify_long(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd,
+template <class SM, int MinBlocks>
+__global__ void __launch_bounds__(2 * SM::H, MinBlocks) k_classify_long(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd,
                                                                      const uint32_t* list, const unsigned* list_n,
                                                                      unsigned* cursor, uint32_t* next,
                                                                      unsigned* next_n, unsigned* n_small,
                                                                      unsigned* n_large) {
   extern __shared__ __align__(16) uint8_t dsm[];
-  LongSmem& S = *reinterpret_cast<LongSmem*>(dsm);
+  SM& S = *reinterpret_cast<SM*>(dsm);
   __shared__ uint32_t s_item;
   const uint32_t n = *list_n;
   if (blockIdx.x >= n) return;
@@ -1075,10 +1077,10 @@ static int occupancy(const void* fn, int threads, size_t smem) {
 static Shapes shapes(const mg_index* ix) {
   static int occ_dual = 0, occ_second = 0, occ_third = 0, occ_long = 0;
   if (!occ_dual) {
-    cudaFuncSetAttribute(k_classify_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LongSmem));
+    cudaFuncSetAttribute(k_classify_long<LongSmem, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LongSmem));
     occ_second = occupancy((const void*)k_classify_dual_list<128, kW2Warps>, kW2Warps * 32, 0);
     occ_third = occupancy((const void*)k_classify_dual_list<256, kW3Warps>, kW3Warps * 32, 0);
-    occ_long = occupancy((const void*)k_classify_long, 2 * LongSmem::H, sizeof(LongSmem));
+    occ_long = occupancy((const void*)k_classify_long<LongSmem, 4>, 2 * LongSmem::H, sizeof(LongSmem));
     occ_dual = occupancy((const void*)k_classify_dual, kW1Warps * 32, 0);
   }
   const mg_tuning& t = ix->tune;
@@ -1171,7 +1173,7 @@ int ensure_workspace(Workspace& w, uint64_t n_reads, uint64_t n_bases, bool host
   }
   if (w.stage.alloc(n_reads * kSlots * sizeof(mg_candidate) + 16) ||
       w.arena.alloc(arena_cap * sizeof(mg_candidate)) || w.ctr.alloc(256) ||
-      w.ovf.alloc(5 * (n_reads + 4) * 4 + 16) || w.sums.alloc(((n_reads + kScanBlock - 1) / kScanBlock + 1) * 8))
+      w.ovf.alloc(6 * (n_reads + 4) * 4 + 16) || w.sums.alloc(((n_reads + kScanBlock - 1) / kScanBlock + 1) * 8))
     return set_error(MG_ERR_OOM, "staging buffers");
   const WsLayout l3 = ws_layout(kB3Q, kB3Seeds, kB3E, kB3C);
   if (w.gws.alloc(l3.total * kB3Blocks)) return set_error(MG_ERR_OOM, "global workspace");
@@ -1179,8 +1181,8 @@ int ensure_workspace(Workspace& w, uint64_t n_reads, uint64_t n_bases, bool host
 }
 
 // Counters in w_ctr (device): 0 n_cands(u64) | 8 arena_n(u64) | 16 err | 20 work | 28 work2 |
-// 32 n_ovf2 | 36 work3 | 40 total(u64) | 48 n_ovf0 | 56 n_ovf0b | 60 work0b | 64 n_large |
-// 68 work of the long-read tier | 72 n_ovf0c | 76 work0c | 80 n_small | 88 n_ovf3 (the global tier's
+// 32 n_ovf2 | 36 work3 | 40 total(u64) | 48 n_ovf0 | 52 n_rest | 56 n_ovf0b | 60 work0b | 64 n_large |
+// 68 work of the long-read tier | 72 n_ovf0c | 76 work0c | 80 n_small | 84 work of its second class | 88 n_ovf3 (the global tier's
 // leftovers) | 92 work4 | 96 oversize need: most bases, seeds, postings, reads waiting (4 x u32) |
 // reads too long for the dual-strand tiers that the first one met: 24 (64 postings), 112 (128), 116 (256) |
 // 120 blocks done in k_count_scan
@@ -1209,6 +1211,9 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
   b.ovf0b = w.ovf.as<uint32_t>() + 3 * (n + 4);
   b.ovf2 = w.ovf.as<uint32_t>() + 2 * (n + 4);
   unsigned* n_large = (unsigned*)(ctr + 64);  // reads that the long-read tier's whole block could not take
+  uint32_t* rest = w.ovf.as<uint32_t>() + 5 * (n + 4);  // those, for the tier's second class
+  unsigned* n_rest = (unsigned*)(ctr + 52);
+  unsigned* work_rest = (unsigned*)(ctr + 84);
   unsigned* work_long = (unsigned*)(ctr + 68);
   uint32_t* ovf0c = w.ovf.as<uint32_t>() + n + 4;  // the 128-posting tier's leftovers
   unsigned* n_ovf0c = (unsigned*)(ctr + 72);
@@ -1233,7 +1238,8 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
   static bool attr_set = false;
   if (!attr_set) {
     CU(cudaFuncSetAttribute(k_classify_block<kB2Threads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l2.total));
-    CU(cudaFuncSetAttribute(k_classify_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LongSmem)));
+    CU(cudaFuncSetAttribute(k_classify_long<LongSmem, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LongSmem)));
+    CU(cudaFuncSetAttribute(k_classify_long<RestSmem, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RestSmem)));
     attr_set = true;
   }
   const bool tm = ix->timing && ix->events_made;
@@ -1250,12 +1256,15 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
     auto further_tiers = [&](cudaStream_t s) -> int {
       if (tm) CU(cudaEventRecord(ix->ev[2], s));
       if (tm) CU(cudaEventRecord(ix->ev[3], s));
-      if (ix->dix.n_refs <= (1u << 21))
-        k_classify_long<<<grid(sh.long_blocks_per_sm * sms, 1), 2 * LongSmem::H, sizeof(LongSmem), s>>>(
-            ix->dix, b, sd, b.ovf0b, b.n_ovf0b, work_long, b.ovf2, b.n_ovf2, n_small, n_large);
-      else
+      if (ix->dix.n_refs <= (1u << 21)) {
+        k_classify_long<LongSmem, 4><<<grid(sh.long_blocks_per_sm * sms, 1), 2 * LongSmem::H, sizeof(LongSmem), s>>>(
+            ix->dix, b, sd, b.ovf0b, b.n_ovf0b, work_long, rest, n_rest, n_small, n_large);
+        k_classify_long<RestSmem, 2><<<grid(2 * sms, 1), 2 * RestSmem::H, sizeof(RestSmem), s>>>(
+            ix->dix, b, sd, rest, n_rest, work_rest, b.ovf2, b.n_ovf2, nullptr, nullptr);
+      } else {
         k_classify_block<kB2Threads><<<grid(sms, 1), kB2Threads, l2.total, s>>>(
             ix->dix, b, sd, b.ovf0b, b.n_ovf0b, b.work2, b.ovf2, b.n_ovf2, nullptr, l2, c2, 0);
+      }
       if (tm) CU(cudaEventRecord(ix->ev[4], s));
       k_classify_block<kB3Threads><<<grid(kB3Blocks, 1), kB3Threads, 0, s>>>(ix->dix, b, sd, b.ovf2, b.n_ovf2, b.work3, ovf3,
                                                                     n_ovf3, w.gws.as<uint8_t>(), l3, c3, !w.hmode);

@@ -2,7 +2,8 @@
 // bases, or more postings than they hold) and every read of the plain form. A block takes a read;
 // its two halves of H threads take one strand each, side by side, and synchronise on a named
 // barrier each; a strand that does not fit its half's share of the shared memory makes the whole
-// block take the strands in turn with all of it. What does not fit then goes to the next tier.
+// block take the strands in turn with all of it. What does not fit then goes to a second class of block
+// (RestSmem), and what that does not hold to the next tier.
 //
 // The strand's bases are hashed from global memory (a seed's window is five aligned words), so
 // shared memory holds postings only, 8 bytes each plus a 2-byte index, in seed order.
@@ -13,7 +14,9 @@
 //                      references with a link matter, and a strand without any is done. The search
 //                      goes through the previous seed's bucket from just before the posting's own
 //                      place in its bucket: copies of a repeat keep their order from bucket to bucket,
-//                      so they meet in a few comparisons; buckets of random hits are one or two long.
+//                      so they meet in a few comparisons; buckets of random hits are one or two long. The
+//                      worst, neighbouring buckets of 2,000 (4,000) postings with no reference in common,
+//                      takes 2.2 (9.1) us a read in a batch of 1,000; the global-memory tier 11 (26) us.
 //   occurrence filter  per linked reference a bitmap of the found indices where it occurs; its longest
 //                      run of ones is occMax; references with max(2, hs - 1) or more stay (:2115)
 //   order              the kept postings by reference, each one's in seed order (a posting's place is
@@ -39,14 +42,18 @@ namespace mg {
 constexpr uint32_t kLgEmpty = 0xFFFFFFFFu;
 constexpr uint32_t kLgKeepAll = 64;       // see long_strand's `wide`
 constexpr uint32_t kRankMax = 128;        // postings of a reference that a warp ranks
-constexpr uint32_t kLgWork = 1u << 21;    // most comparisons of the link search (sum of squared buckets)
+constexpr uint32_t kNone = 0xFFFFu;       // no link (long_strand, step 2)
+constexpr uint32_t kRunEnd = 0x8000u;     // a run's length in place of its last posting's link
 
 // Shared memory of a block: two halves of H threads, each with room for E postings, NS seeds and RM
 // kept references per strand (RT table slots); the whole block uses both shares of the postings and
-// seeds for one strand.
-template <int H_, int E_, int NS_, int RT_, int RM_>
+// seeds for one strand. Rest: the class for what the others leave, which takes strands on the whole
+// block only, and the keep rule ahead of the table (keep_by_runs).
+template <int H_, int E_, int NS_, int RT_, int RM_, bool Rest_ = false>
 struct alignas(16) LongSm {
   static constexpr int H = H_, E = E_, NS = NS_, RT = RT_, RM = RM_;
+  static constexpr bool Rest = Rest_;
+  static constexpr uint32_t kIdBits = RM > 126 ? 8 : 7, kNoId = (1u << kIdBits) - 1;  // a reference's order of insertion
   static constexpr int NSP = NS + 1, NW = (NS + 31) / 32, BW = E / 64;  // BW: words of E / 2 bits
   struct Half {
     unsigned long long sumr[RM];  // sums of a candidate's runs; before: the linked references' best
@@ -75,18 +82,22 @@ struct alignas(16) LongSm {
   Half h[2];
   mg_candidate cb[2][RM];
   uint8_t comp[256];  // complement(upper(byte)), 0 where there is none
-  static_assert(E % 64 == 0 && E % 4 == 0 && NSP % 2 == 0 && 2 * E <= 8192 && NS <= E / 2 && 2 * NS <= 2047 && RT <= 256 && RM < 127, "sizes");
+  static_assert(E % 64 == 0 && E % 4 == 0 && NSP % 2 == 0 && 2 * E <= 8192 && NS <= E / 2 && 2 * NS <= 2047 && RM < kNoId && 3 * RM <= E / 2 && (!Rest || 2 * E / 32 <= RT), "sizes");
   static_assert(RM * 8 >= 2 * (RM + 1), "tables over the sums");
 };
 
 // The classes of reads: the batched forms' tier (reads to 20,480 bases and 4,096 postings per strand)
 // with four blocks per SM, and the plain form's kernel, one block of two warps per read, up to 15 per
 // SM (11,000 reads of 150 bases: 97 us; a block of 256 threads per read with two bitonic sorts per
-// strand, the form before, 1,010 us; room for 256 postings instead of 512 makes no difference).
+// strand, the form before, 1,010 us; room for 256 postings instead of 512 makes no difference). Then
+// what the first leaves: two blocks per SM, 8,192 postings (4,096 kept), 2,046 seeds (reads of 20,480
+// bases down to k = 20) and 224 kept references, whatever the number of linked ones.
 using LongSmem = LongSm<128, 2048, 703, 256, 88>;
 using PlainSmem = LongSm<32, 512, 255, 64, 32>;
+using RestSmem = LongSm<128, 4096, 1023, 512, 224, true>;
 constexpr uint32_t kLgQ = 20480;
 static_assert(4 * (sizeof(LongSmem) + 1024) <= 233472, "four blocks per SM");
+static_assert(2 * (sizeof(RestSmem) + 1024) <= 233472, "two blocks per SM");
 
 __device__ __forceinline__ uint32_t lg_mix(uint32_t x) { return (x * 2654435761u) ^ (x >> 15); }
 
@@ -239,6 +250,122 @@ __device__ __forceinline__ uint32_t warp_longest_run(const uint32_t* bm, uint32_
   return __shfl_sync(0xffffffffu, best, 0);
 }
 
+// A posting under the found seed before posting i's (x = rs[i]) with its reference; kNone: there is none
+// (or !on). The warp reconverges.
+__device__ __forceinline__ uint32_t link_of(const uint32_t* rs, const uint16_t* st, const uint16_t* cn,
+                                            const uint32_t* fm, uint32_t i, uint32_t x, bool on) {
+  const uint32_t j = x & 2047u;
+  uint32_t w = j >> 5, m = on ? fm[w] & ((1u << (j & 31u)) - 1u) : 0u;
+#pragma unroll 1
+  while (!m && w && on) m = fm[--w];
+  uint32_t a = 0, c = 0, t = 0, at = kNone;
+  if (m) {
+    const uint32_t pj = w * 32 + 31 - __clz(m);
+    a = st[pj];
+    c = cn[pj];
+    t = i - st[j];  // a stray hit in either bucket shifts the copies by one
+    t = t < 2 ? 0 : t - 2;
+    if (t >= c) t = 0;
+  }
+#pragma unroll 1
+  for (uint32_t n = 0; n < c && at == kNone; n++) {
+    if ((rs[a + t] ^ x) < 2048u) at = a + t;
+    if (++t == c) t = 0;
+  }
+  __syncwarp();
+  return at;
+}
+
+// A reference (on) into the strand's table, with the next number; S.over: more than RM. The warp
+// reconverges.
+template <class SM>
+__device__ __forceinline__ void add_ref(SM& S, int half, uint32_t ref, bool on) {
+  typename SM::Half& T = S.h[half];
+  uint32_t s = lg_mix(ref) & (SM::RT - 1), left = on ? (uint32_t)SM::RT : 0u;  // each slot once
+#pragma unroll 1
+  while (left) {
+    uint32_t old = *(volatile uint32_t*)&T.rt[s];
+    if (old == kLgEmpty && !*(volatile uint32_t*)&S.over[half]) {  // the table stays free to end probes
+      old = atomicCAS(&T.rt[s], kLgEmpty, ref);
+      if (old == kLgEmpty) {
+        const uint32_t id = atomicAdd(&S.n_rt[half], 1u);
+        if (id < (uint32_t)SM::RM) {
+          T.rid[s] = (uint8_t)id;
+          T.sumc[id] = ref;
+        } else {
+          S.over[half] = 1;
+        }
+      }
+    }
+    left = old == ref || old == kLgEmpty ? 0u : left - 1;
+    s = (s + 1) & (SM::RT - 1);
+  }
+  __syncwarp();
+}
+
+// The keep rule ahead of the table, on the whole block, for a strand of ne postings with more linked
+// references than the table or the bitmaps hold: most are copies of a repeat that the rule drops beside
+// the strand's own reference. A posting's links, followed back, are the occurrence run that ends at it;
+// only references with a run long enough go to the table. Returns how many (above RM: too many), the
+// longest run at each of them in `best`. Reads of 250 bases on the flank of a segment with 100 (200)
+// copies and inside it, 10,000 each: 1.2 (3.0) and 2.2 (3.7) ms; through the global-memory tier, which
+// took what LongSmem does not hold, 28 (67) and 112 (237) ms. 2,000 reads of 16 kb across several
+// segments of 30 copies: 1.0 ms, 28.5 ms so. Not in the first class: there the call's registers
+// spill in the common strands (20,000 reads of 1-20 kb: 1.70 ms, 1.67 ms without).
+template <class SM>
+__device__ __forceinline__ uint32_t keep_by_runs(SM& S, uint32_t ne) {
+  constexpr uint32_t G = 2 * SM::H, kE = 2 * SM::E, kRT = SM::RT;
+  const uint32_t tid = threadIdx.x;
+  const uint32_t* rs = S.rs;
+  const uint16_t* st = S.pool + kE;
+  const uint16_t* cn = st + 2 * SM::NSP;
+  typename SM::Half& T = S.h[0];
+  uint16_t* ln = S.pool;     // each posting's link, over sx and kl; then at a run's last posting its length
+  uint32_t* on = S.h[1].rt;  // postings that a run goes on from, a bit each (the other half's table is free)
+  uint16_t* best = reinterpret_cast<uint16_t*>(T.sumr);
+  __syncthreads();  // every thread has read the table's count
+#pragma unroll 1
+  for (uint32_t i = tid; i < kE / 32; i += G) on[i] = 0;
+#pragma unroll 1
+  for (uint32_t i = tid; i < kRT; i += G) T.rt[i] = kLgEmpty;
+  if (tid == 0) {
+    S.n_rt[0] = 0;
+    S.over[0] = 0;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t i0 = 0; i0 < ne; i0 += G) {
+    const uint32_t i = i0 + tid, l = link_of(rs, st, cn, S.fm, i, i < ne ? rs[i] : 0u, i < ne);
+    if (i < ne) ln[i] = (uint16_t)l;
+    if (l != kNone) atomicOr(&on[l >> 5], 1u << (l & 31u));
+  }
+  __syncthreads();
+  uint32_t hs = 0;
+#pragma unroll 1
+  for (uint32_t i = tid; i < ne; i += G) {
+    uint32_t p = ln[i], len = 1;
+    if (p == kNone || ((on[i >> 5] >> (i & 31u)) & 1u)) continue;
+#pragma unroll 1
+    for (; p != kNone; p = ln[p]) len++;  // fewer steps than seeds: a link leads to an earlier one
+    ln[i] = (uint16_t)(kRunEnd | len);    // no other run passes here
+    hs = max(hs, len);
+  }
+  hs = __reduce_max_sync(0xFFFFFFFFu, hs);
+  if ((tid & 31u) == 0) S.red[0][0][tid >> 5] = hs;
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t w = 0; w < G / 32; w++) hs = max(hs, S.red[0][0][w]);
+#pragma unroll 1
+  for (uint32_t i0 = 0; i0 < ne; i0 += G) {
+    const uint32_t i = i0 + tid, v = i < ne ? ln[i] : kNone;
+    add_ref(S, 0, i < ne ? rs[i] >> 11 : 0u, v != kNone && (v & kRunEnd) && (v & (kRunEnd - 1)) >= max(2u, hs - 1));
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (uint32_t id = tid; id < (uint32_t)SM::RM; id += G) best[id] = (uint16_t)hs;
+  return S.n_rt[0];
+}
+
 // One strand of a read (raw bytes, L of them, no byte without a complement; acgt: all of them letters
 // of ACGT in either case) on G threads with room for kE postings and kNS seeds: half `half` of the
 // block (G = H), or all of it (whole: G = 2 H, half 0). On kStrandOk the strand's *n_out scored candidates
@@ -297,7 +424,6 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   //    the group's cursor, so nothing waits for another warp and the postings lie in no order.
   uint16_t* xl = kl;                              // seeds with more than a slot's postings (at most kE / 8)
   uint32_t* xo = reinterpret_cast<uint32_t*>(sx);  // their first posting in the index
-  uint32_t sq2 = 0;                                // this thread's seeds' squared bucket sizes
 #pragma unroll 1
   for (uint32_t j0 = 0; j0 < ns; j0 += 2 * G) {
     uint4 v0[2], v1[2];
@@ -347,7 +473,6 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
       }
       const uint32_t fb = __ballot_sync(FULL, full > 0 || h == ix.empty_hash);
       const uint32_t n = min(full, kE + 1);
-      sq2 += n * n;
       uint32_t x = n;
       for (int t = 1; t < 32; t <<= 1) {
         const uint32_t y = __shfl_up_sync(FULL, x, t);
@@ -394,17 +519,10 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
       }
     }
   }
-  for (int o = 16; o; o >>= 1) sq2 += min(__shfl_xor_sync(FULL, sq2, o), kLgWork);  // far below 2^32
-  if (lane == 0) red[0][warp] = min(sq2, kLgWork + 1);
   lg_sync<SM::H>(bar);
   const uint32_t ne = S.ne[half], nx = S.nx[half];
-  {
-    uint32_t work = 0;
-#pragma unroll 1
-    for (uint32_t w = 0; w < kW; w++) work += red[0][w];
-    if (ne > kE || work > kLgWork) return kStrandOverflow;  // group-uniform
-    if (ne == 0) return kStrandOk;  // nothing found: the reference skips the strand
-  }
+  if (ne > kE) return kStrandOverflow;  // group-uniform
+  if (ne == 0) return kStrandOk;        // nothing found: the reference skips the strand
   if (warp == kW - 1) {  // found seeds before each word: at most 64 words, two a lane
     const uint32_t nw = (ns + 31) >> 5;
     const uint32_t c0 = 2 * lane < nw ? __popc(fm[2 * lane]) : 0u, c1 = 2 * lane + 1 < nw ? __popc(fm[2 * lane + 1]) : 0u;
@@ -436,61 +554,28 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   // 2. the linked references (the warps reconverge between the two searches)
 #pragma unroll 1
   for (uint32_t i0 = 0; i0 < ne; i0 += G) {
-    const uint32_t i = i0 + tid, x = i < ne ? rs[i] : 0u, j = x & 2047u;
-    uint32_t w = j >> 5, m = i < ne ? fm[w] & ((1u << (j & 31u)) - 1u) : 0u;
-#pragma unroll 1
-    while (!m && w && i < ne) m = fm[--w];
-    uint32_t a = 0, c = 0, t = 0;
-    if (m) {
-      const uint32_t pj = w * 32 + 31 - __clz(m);
-      a = st[pj];
-      c = cn[pj];
-      t = i - st[j];  // a stray hit in either bucket shifts the copies by one
-      t = t < 2 ? 0 : t - 2;
-      if (t >= c) t = 0;
-    }
-    bool linked = false;
-#pragma unroll 1
-    for (uint32_t n = 0; n < c && !linked; n++) {
-      linked = (rs[a + t] ^ x) < 2048u;
-      if (++t == c) t = 0;
-    }
-    __syncwarp();
-    const uint32_t ref = x >> 11;
-    uint32_t s = lg_mix(ref) & (kRT - 1), left = linked ? kRT : 0u;  // each slot once
-#pragma unroll 1
-    while (left) {
-      uint32_t old = *(volatile uint32_t*)&T.rt[s];
-      if (old == kLgEmpty && !*(volatile uint32_t*)&S.over[half]) {  // the table stays free to end probes
-        old = atomicCAS(&T.rt[s], kLgEmpty, ref);
-        if (old == kLgEmpty) {
-          const uint32_t id = atomicAdd(&S.n_rt[half], 1u);
-          if (id < kRM) {
-            T.rid[s] = (uint8_t)id;
-            iref[id] = ref;
-          } else {
-            S.over[half] = 1;
-          }
-        }
-      }
-      left = old == ref || old == kLgEmpty ? 0u : left - 1;
-      s = (s + 1) & (kRT - 1);
-    }
-    __syncwarp();
+    const uint32_t i = i0 + tid, x = i < ne ? rs[i] : 0u;
+    const bool linked = link_of(rs, st, cn, fm, i, x, i < ne) != kNone;
+    add_ref(S, half, x >> 11, linked);
   }
   lg_sync<SM::H>(bar);
-  const uint32_t R = S.n_rt[half];
+  uint32_t R = S.n_rt[half];
   if (R == 0) return kStrandOk;  // no reference at two found seeds in a row: no candidate
   // the bitmaps (R of nfw words) and, behind them, the ones before each word (R nfw half-words) lie over sx
-  if (R > kRM || 3 * R * nfw > kE / 2) return kStrandOverflow;
+  if (R > kRM || 3 * R * nfw > kE / 2) {
+    if (!SM::Rest) return kStrandOverflow;
+    R = keep_by_runs(S, ne);
+    if (R > kRM) return kStrandOverflow;
+  }
+  const bool nobm = SM::Rest && 3 * R * nfw > kE / 2;  // no room for bitmaps: the kept postings are counted and ranked one by one
   // 3. occurrence filter; from here on the postings hold, in place of the refID, its reference's order
   //    of insertion (kNoId: not linked, not needed any more)
-  constexpr uint32_t kNoId = 127;
+  constexpr uint32_t kNoId = SM::kNoId, kPlace = 11 + SM::kIdBits;  // id << 11 | seed, and a place above it
   uint32_t* bm = reinterpret_cast<uint32_t*>(sx);
   uint16_t* pw = sx + 2 * R * nfw;
 #pragma unroll 1
-  for (uint32_t i = tid; i < R * nfw; i += G) bm[i] = 0;
-  if (tid == 0) S.dup[half] = 0;
+  for (uint32_t i = tid; i < R * nfw && !nobm; i += G) bm[i] = 0;
+  if (tid == 0) S.dup[half] = nobm;
   lg_sync<SM::H>(bar);
   const uint32_t only = iref[0];
 #pragma unroll 1
@@ -512,7 +597,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     __syncwarp();
     if (i < ne) {
       rs[i] = (id << 11) | j;
-      if (id != kNoId) {
+      if (id != kNoId && !nobm) {
         const uint32_t f = fp[j >> 5] + __popc(fm[j >> 5] & ((1u << (j & 31u)) - 1u)), bit = 1u << (f & 31u);
         if (atomicOr(&bm[id * nfw + (f >> 5)], bit) & bit) S.dup[half] = 1;  // twice under one seed
       }
@@ -526,7 +611,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
       T.cnt[id] = (uint16_t)__popc(bm[id]);
       pw[id] = 0;
     }
-  } else {
+  } else if (!nobm) {
 #pragma unroll 1
     for (uint32_t id = warp; id < R; id += kW) {
       uint32_t n;
@@ -562,7 +647,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
 #pragma unroll 1
   for (uint32_t i = tid; i < kRM; i += G) T.segmax[i] = 0;
   lg_sync<SM::H>(bar);
-  auto rank_of = [&](uint32_t x) -> uint32_t { return T.rk[(x >> 11) & 127u]; };  // of a linked posting
+  auto rank_of = [&](uint32_t x) -> uint32_t { return T.rk[(x >> 11) & kNoId]; };  // of a linked posting
   // 4. the kept postings in (refID, position, seed) order, as indices in sx[0 .. T2)
   auto key_of = [&](uint32_t i) { return ((uint64_t)ps[i] << 11) | (rs[i] & 2047u); };
   uint32_t T2 = 0;
@@ -594,7 +679,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
 #pragma unroll 1
     for (uint32_t i = tid; i < ne; i += G) {  // a posting's place in its range goes beside its id
       const uint32_t x = rs[i];
-      if ((x >> 11) != kNoId && rank_of(x) != kNoId) rs[i] = x | (atomicAdd(&bfill[x >> 11], 1u) << 18);
+      if ((x >> 11) != kNoId && rank_of(x) != kNoId) rs[i] = x | (atomicAdd(&bfill[x >> 11], 1u) << kPlace);
     }
     lg_sync<SM::H>(bar);
 #pragma unroll 1
@@ -620,11 +705,11 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   lg_sync<SM::H>(bar);
 #pragma unroll 1
   for (uint32_t i = tid; i < ne; i += G) {  // into the ranges, in seed order unless dup
-    const uint32_t x = rs[i], id = (x >> 11) & 127u;
+    const uint32_t x = rs[i], id = (x >> 11) & kNoId;
     if (id == kNoId) continue;
     const uint32_t b = T.rk[id];
     if (b == kNoId) continue;
-    uint32_t at = x >> 18;
+    uint32_t at = x >> kPlace;
     if (!dup) {
       const uint32_t j = x & 2047u, f = fp[j >> 5] + __popc(fm[j >> 5] & ((1u << (j & 31u)) - 1u));
       const uint32_t w = id * nfw + (f >> 5);
@@ -700,7 +785,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
     if (i < T2 && i > 0) {
       const uint32_t a = sx[i - 1], b = sx[i];
       // one reference and seed + 1: one addition on the packed word
-      const uint32_t xa = rs[a] & 0x3FFFFu, xb = rs[b] & 0x3FFFFu;
+      const uint32_t xa = rs[a] & ((1u << kPlace) - 1u), xb = rs[b] & ((1u << kPlace) - 1u);
       start = !((uint64_t)ps[a] + step == ps[b] && xa + 1u == xb && (xb & 2047u) != 0);
     }
     const uint32_t w = __ballot_sync(FULL, start);
@@ -916,8 +1001,8 @@ __device__ bool process_read_long(const DevIndex& ix, const BatchDev& b, uint32_
   bool wide = false, over = false;
   // first the strands side by side, then, when one does not fit its half, in turn on the whole block
 #pragma unroll 1
-  for (int pass = 0; pass < 3; pass++) {
-    const bool whole = pass > 0;
+  for (int pass = SM::Rest ? 1 : 0; pass < 3; pass++) {
+    const bool whole = SM::Rest || pass > 0;
     const int half = whole ? 0 : threadIdx.x / H, strand = whole ? pass - 1 : half;
     uint32_t n1;
     float h1;

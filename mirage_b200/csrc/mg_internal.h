@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <mutex>
 #include <string>
+#include <utility>
 
 #include "../../include/mirage_b200.h"
 #include "mg_device.cuh"
@@ -14,9 +15,20 @@
 
 namespace mg {
 
+// A device allocation, freed with its owner. (cudaFree waits for the work in flight that uses it.)
 struct DevBuf {
   void* p = nullptr;
   size_t n = 0;
+  DevBuf() = default;
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  DevBuf(DevBuf&& o) noexcept { std::swap(p, o.p), std::swap(n, o.n); }
+  DevBuf& operator=(DevBuf&& o) noexcept {
+    std::swap(p, o.p);
+    std::swap(n, o.n);
+    return *this;
+  }
+  ~DevBuf() { release(); }
   int alloc(size_t bytes) {
     if (bytes <= n && p) return 0;
     if (p) cudaFree(p);

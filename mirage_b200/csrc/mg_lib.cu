@@ -1395,7 +1395,6 @@ static void add_slabs(Workspace& w, uint32_t n_huge) {
   const int slabs = take_slabs(want, w.hslabs + 1, [&](int n) { return more.alloc(l.total * (size_t)n) == 0; });
   if (slabs) {
     std::swap(w.hws, more);
-    more.release();
     w.hslabs = slabs;
   }
   w.hshort = slabs != want;
@@ -2098,8 +2097,8 @@ int mg_score_candidates(mg_index* ix, uint64_t n_strands, const uint64_t* q_off,
   }
   const uint64_t hw = (maxL + 31) / 32 + 1;
   // The device buffers are pieces of one that the index keeps and grows to its largest call: eleven
-  // allocations and frees on every call, and the device-wide waits of the frees, took two thirds of it
-  // (20,000 strands with 27,000 candidates: 1.6 ms, or 4.9 ms when the driver unmapped their memory; 0.69 ms now).
+  // allocations on every call took half of it and more (20,000 strands with 27,000 candidates: 1.6 ms, on
+  // some calls 4.9 ms; 0.69 ms now).
   DevPiece dq, db, dr, drun, dcs, dro, dsc, dpc, drl, dhit, derr;
   uint64_t need = 0;
   auto piece = [&](DevPiece& v, uint64_t bytes) {

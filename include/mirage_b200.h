@@ -178,9 +178,12 @@ int mg_gather_bandwidth(int device, uint64_t buffer_bytes, double* gbs);
 int mg_last_kernel_times(mg_index* ix, float* ms5);
 /* Diagnostic: how many reads each tier of the last batched call run in one piece (the device
  * form, or host buffers too few to chunk) handed on: [the 64-, 128- and 256-posting dual-strand
- * tiers, the last of these again (a general warp tier, now part of the long-read tier), the long-read
- * tier's half-blocks and its whole block, to its second class (both also count a strand that keeps every reference and was
- * finished outside their tables), the long-read tier in all] (the last goes to the global-memory tier). With first_tier 2 or 3 the tiers before it count 0. */
+ * tiers, the last of these again (a general warp tier, now part of the long-read tier), the
+ * half-blocks of the long-read tier's first class, its whole blocks (what these hand on goes to the
+ * second class), the long-read tier in all (what it hands on goes to the global-memory tier)]. With
+ * first_tier 2 or 3 the tiers before it count 0. The two entries of the first class also count the
+ * reads with a strand whose longest occurrence run is 2, which keeps every reference with a posting,
+ * on more than 64 postings and with a diagonal run: these are not handed on. */
 int mg_last_tier_counts(mg_index* ix, uint32_t* counts7);
 int mg_bucket_sizes(mg_index* ix, const uint32_t* hashes, uint32_t* counts, uint64_t n);
 

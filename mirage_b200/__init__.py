@@ -340,7 +340,8 @@ class Index:
         return ms
 
     def last_tier_counts(self) -> dict:
-        """Reads each tier of the last one-piece batched call handed on (mg_last_tier_counts)."""
+        """Reads each tier of the last one-piece batched call handed on; "long_small" and "long_large" also
+        count some reads that were finished there (mg_last_tier_counts)."""
         c = np.zeros(7, np.uint32)
         _check(lib().mg_last_tier_counts(self.h, c.ctypes.data), "mg_last_tier_counts")
         names = ["dual64", "dual128", "dual256", "warp", "long_small", "long_large", "block"]

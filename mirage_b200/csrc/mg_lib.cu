@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(2 * SM::H, MinBlocks) k_classify_long(const __
   const uint32_t n = *list_n;
   if (blockIdx.x >= n) return;
   for (int c = threadIdx.x; c < 256; c += blockDim.x) S.comp[c] = complement_dev(upper_dev((uint8_t)c));
-  if (threadIdx.x == 0) S.handed = 0;
+  if (threadIdx.x == 0) S.keeps_all = 0;
   uint32_t ahead = threadIdx.x == 0 ? atomicAdd(cursor, 1u) : 0u;
   for (;;) {
     if (threadIdx.x == 0) s_item = ahead;
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(2 * PlainSmem::H) k_classify_plain(const __gri
                                                                     unsigned* next_n) {
   __shared__ PlainSmem S;
   for (int c = threadIdx.x; c < 256; c += blockDim.x) S.comp[c] = complement_dev(upper_dev((uint8_t)c));
-  if (threadIdx.x == 0) S.handed = 0;
+  if (threadIdx.x == 0) S.keeps_all = 0;
   __syncthreads();
   const uint32_t r = blockIdx.x;
   if (!process_read_long(ix, b, r, S, sd.stage, sd.arena, sd.arena_cap, sd.arena_n, b.err, nullptr, nullptr)) {
@@ -1909,7 +1909,8 @@ int mg_last_tier_counts(mg_index* ix, uint32_t* counts7) {
   // the lists' counters (run_pipeline): left by the 64-, 128- and 256-posting dual tiers (with the reads
   // too long for them, which skip the rest; the tiers not run count what passes them; the last also as
   // the general warp tier's entry, which has no tier of its own any more), by the long-read tier's
-  // half-blocks and its whole block, and in all for the global-memory tier
+  // half-blocks and its whole block (both with the reads that keep every reference, long_strand), and in
+  // all for the global-memory tier
   auto u32 = [&](int o) {
     uint32_t v;
     std::memcpy(&v, h + o, 4);

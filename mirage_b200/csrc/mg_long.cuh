@@ -40,7 +40,7 @@
 namespace mg {
 
 constexpr uint32_t kLgEmpty = 0xFFFFFFFFu;
-constexpr uint32_t kLgKeepAll = 64;       // see long_strand's `wide`
+constexpr uint32_t kLgKeepAll = 64;       // see long_strand's `keeps_all`
 constexpr uint32_t kRankMax = 128;        // postings of a reference that a warp ranks
 constexpr uint32_t kNone = 0xFFFFu;       // no link (long_strand, step 2)
 constexpr uint32_t kRunEnd = 0x8000u;     // a run's length in place of its last posting's link
@@ -75,7 +75,7 @@ struct alignas(16) LongSm {
   uint16_t fp[2 * NW];  // found seeds before each word of fm
   uint32_t bk[2 * BW];  // starts of diagonal runs
   uint32_t red[2][2][2 * H / 32];
-  uint32_t ne[2], nx[2], n_rt[2], over[2], dup[2], n_ends[2], n_out[2], handed;
+  uint32_t ne[2], nx[2], n_rt[2], over[2], dup[2], n_ends[2], n_out[2], keeps_all;
   float hi[2];
   int status[2];
   uint32_t cand_at, ahead;
@@ -370,8 +370,9 @@ __device__ __forceinline__ uint32_t keep_by_runs(SM& S, uint32_t ne) {
 // of ACGT in either case) on G threads with room for kE postings and kNS seeds: half `half` of the
 // block (G = H), or all of it (whole: G = 2 H, half 0). On kStrandOk the strand's *n_out scored candidates
 // are in cb, in ascending refID, and *highest is its HighestScore. kStrandOverflow: it does not fit.
-// *wide: the keep rule keeps more references than a table of kLgKeepAll postings' worth (hs = 2
-// keeps every reference with a posting) and the strand has a diagonal run.
+// *keeps_all: the keep rule keeps every reference with a posting (hs = 2), the strand has more than
+// kLgKeepAll postings and a diagonal run. Only counted (mg_last_tier_counts): such a strand has its
+// candidates among the linked references like any other.
 // One instance for both, and loops kept rolled: the code runs through once per strand, so that its
 // size is paid in instruction fetches. With an instance each and the compiler's unrolling it was
 // 355 KB, and four blocks per SM slowed each other from 64,000 to 119,000 cycles a read (20,000 reads
@@ -379,7 +380,7 @@ __device__ __forceinline__ uint32_t keep_by_runs(SM& S, uint32_t ne) {
 template <class SM>
 __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* raw, uint32_t L, int strand, bool acgt,
                                            SM& S, bool whole, int half, mg_candidate* cb, int* err, uint32_t* n_out,
-                                           float* highest, bool* wide) {
+                                           float* highest, bool* keeps_all) {
   constexpr uint32_t kRT = SM::RT, kRM = SM::RM;
   constexpr unsigned FULL = 0xffffffffu;
   const uint32_t sh = whole ? 1u : 0u;  // twice the threads and the room
@@ -809,7 +810,7 @@ __device__ __forceinline__ int long_strand(const DevIndex& ix, const uint8_t* ra
   for (uint32_t b = lane; b < nk; b += 32) M = max(M, T.segmax[b]);
   M = __reduce_max_sync(FULL, M);
   if (M < 2) return kStrandOk;  // Analyser.cpp:2402
-  *wide = hs == 2 && ne > kLgKeepAll;
+  *keeps_all = hs == 2 && ne > kLgKeepAll;
   // 6. candidates: the kept references whose longest run is M, in rank order (every warp has the
   //    masks); the walks of all their runs, a run end a thread, summed per candidate, as many
   //    candidates at a time as their coverage bitmaps have room
@@ -967,8 +968,8 @@ __device__ int read_letters(const uint8_t* raw, uint32_t L, const SM& S) {
 }
 
 // Both strands of read r, the strand merge and the staging write; false when the read must go to the
-// next tier. n_small, n_large (optional): counters of the reads that the halves, and the block with
-// its table of kept references, could not take. ahead (thread 0's): the entry of list that the block
+// next tier. n_small, n_large (optional): counters of the reads that the halves, and the whole block,
+// could not take, and of those with a strand that keeps every reference (long_strand). ahead (thread 0's): the entry of list that the block
 // takes next; while the first warp writes this read's result, the last one asks for that read's bases.
 template <class SM>
 __device__ bool process_read_long(const DevIndex& ix, const BatchDev& b, uint32_t r, SM& S, mg_candidate* stage,
@@ -998,7 +999,7 @@ __device__ bool process_read_long(const DevIndex& ix, const BatchDev& b, uint32_
   int err = 0;
   uint32_t n[2] = {0, 0};
   float h[2] = {-1.0f, -1.0f};
-  bool wide = false, over = false;
+  bool keeps_all = false, over = false;
   // first the strands side by side, then, when one does not fit its half, in turn on the whole block
 #pragma unroll 1
   for (int pass = SM::Rest ? 1 : 0; pass < 3; pass++) {
@@ -1013,7 +1014,7 @@ __device__ bool process_read_long(const DevIndex& ix, const BatchDev& b, uint32_
       S.status[strand] = s;
       S.n_out[strand] = n1;
       S.hi[strand] = h1;
-      if (w) S.handed = 1;  // a strand outside the kept-reference tables, finished here
+      if (w) S.keeps_all = 1;
       if (threadIdx.x == 0) S.ahead = ahead;
     }
     __syncthreads();
@@ -1028,14 +1029,14 @@ __device__ bool process_read_long(const DevIndex& ix, const BatchDev& b, uint32_
       (strand ? n[1] : n[0]) = S.n_out[strand];
       (strand ? h[1] : h[0]) = S.hi[strand];
     }
-    wide = S.handed != 0;
+    keeps_all = S.keeps_all != 0;
     __syncthreads();
-    if (pass == 0 && threadIdx.x == 0 && n_small && (over || wide)) atomicAdd(n_small, 1u);
+    if (pass == 0 && threadIdx.x == 0 && n_small && (over || keeps_all)) atomicAdd(n_small, 1u);
     if (over == whole) break;  // both strands done on the halves, or one does not fit at all
-    if (pass == 0 && threadIdx.x == 0) S.handed = 0;
+    if (pass == 0 && threadIdx.x == 0) S.keeps_all = 0;
   }
-  if (threadIdx.x == 0) S.handed = 0;
-  if (threadIdx.x == 0 && n_large && (over || wide)) atomicAdd(n_large, 1u);
+  if (threadIdx.x == 0) S.keeps_all = 0;
+  if (threadIdx.x == 0 && n_large && (over || keeps_all)) atomicAdd(n_large, 1u);
   if (err) atomicOr(errw, err);  // any thread's: the scoring lanes record bits per thread
   if (over) return false;
   // the strand merge (Analyser.cpp:592-611), the log skip rule (:388) and the staging write

@@ -1314,10 +1314,11 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
       const int rc = further_tiers(w.side);
       if (rc) return rc;
       CU(cudaEventRecord(w.join, w.side));
-      // 32 reads to a warp when they fill the GPU; fewer for a batch that leaves warps idle, so that its
-      // walks, a record per lane, take one round each (20,011 reads: 26 us with 32, 18 us with 8;
-      // 1 M reads: 222 us with 32)
-      const uint32_t per_warp = n < 65536 ? 8 : 32, per_block = kFinThreads / 32 * per_warp;
+      // 32 reads to a warp share one round of walks, a record per lane; fewer make more and shorter rounds,
+      // which pays while the batch leaves warps idle. A batch of 75-300 bases with 8 and with 32: 20,011
+      // reads 91.6 and 94.6 us, 32,768 reads 110 and 114 us; 65,536 reads 157 and 147 us, 131,072 reads
+      // 243 and 212 us (16 lie between, but for 143 us at 65,536)
+      const uint32_t per_warp = n < 49152 ? 8 : 32, per_block = kFinThreads / 32 * per_warp;
       k_finish_dual<<<(unsigned)std::min<uint64_t>((n + per_block - 1) / per_block,
                                                    (uint64_t)sms * sh.finish_blocks_per_sm),
                       kFinThreads, 0, st>>>(ix->dix, b, sd, per_warp);

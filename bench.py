@@ -47,7 +47,7 @@ SEED = 2024
 N_READS = 1_000_000
 # kernels one batched call launches: dual-strand tier, second dual-strand tier (its leftovers), the
 # finishing pass, long-read tier (two classes), global tier, candidate counts and their scan, scatter (an index whose
-# reads start at the second tier launches the third instead of the first; batches of up to 2,048 reads
+# reads start at the second tier launches the third instead of the first; batches of up to 1,024 reads
 # launch one kernel for the last two)
 LAUNCHES_PER_BATCH = 8
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_classify_dual launch on the

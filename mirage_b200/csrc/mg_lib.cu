@@ -599,34 +599,30 @@ __global__ void k_scatter(mg_read_result* reads, uint64_t n, const unsigned long
   if (i < n) scatter_read(reads, i, block_sums[blockIdx.x] + wb + x - v, sd, out, cap, err);
 }
 
-// The whole compaction of a batch of up to kScanSmall reads, one block: a launch instead of two, which
-// is what such a batch waits for.
-constexpr uint64_t kScanSmall = 2 * kScanBlock;
+// The whole compaction of a batch of up to kScanSmall reads, one block with a read a thread: a launch
+// instead of two (a batch of 16 reads: 49.9 us, 53.6 us with two; 1,024 reads: 61.8 and 63.4 us). A second
+// round costs more than the launch (1,500 reads: 67 and 61 us; 2,048: 69 and 64 us).
+constexpr uint64_t kScanSmall = kScanBlock;
 __global__ void __launch_bounds__(kScanBlock) k_compact_small(mg_read_result* reads, uint64_t n, unsigned long long* total,
                                                               StageDev sd, mg_candidate* out, uint64_t cap, int* err) {
   __shared__ unsigned long long s[kScanBlock / 32];
+  const uint64_t i = threadIdx.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned long long carry = 0;
-  for (uint64_t t0 = 0; t0 < n; t0 += kScanBlock) {
-    const uint64_t i = t0 + threadIdx.x;
-    const unsigned long long v = i < n ? (unsigned long long)(reads[i].n_fwd + reads[i].n_rc) : 0ull;
-    unsigned long long x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) s[wid] = x;
-    __syncthreads();
-    unsigned long long wb = 0, tile = 0;
-    for (int w = 0; w < kScanBlock / 32; w++) {
-      wb += w < wid ? s[w] : 0ull;
-      tile += s[w];
-    }
-    if (i < n) scatter_read(reads, i, carry + wb + x - v, sd, out, cap, err);
-    carry += tile;
-    __syncthreads();
+  const unsigned long long v = i < n ? (unsigned long long)(reads[i].n_fwd + reads[i].n_rc) : 0ull;
+  unsigned long long x = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
   }
-  if (threadIdx.x == 0) *total = carry;
+  if (lane == 31) s[wid] = x;
+  __syncthreads();
+  unsigned long long wb = 0, all = 0;
+  for (int w = 0; w < kScanBlock / 32; w++) {
+    wb += w < wid ? s[w] : 0ull;
+    all += s[w];
+  }
+  if (i < n) scatter_read(reads, i, wb + x - v, sd, out, cap, err);
+  if (threadIdx.x == 0) *total = all;
 }
 
 // Index construction: directory from the ascending TOC (dir[h] = first posting of the first

@@ -8,7 +8,7 @@ import mirage_b200 as M
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 49151, 49152, 49153])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 1023, 1024, 1025, 2047, 2048, 2049, 3073, 49151, 49152, 49153])
 def test_batches_of_every_launch_size(golden, n):
     g = golden("uneven_small")
     ix = M.Index(g.image)

@@ -183,7 +183,8 @@ int mg_last_kernel_times(mg_index* ix, float* ms5);
  * second class), the long-read tier in all (what it hands on goes to the global-memory tier)]. With
  * first_tier 2 or 3 the tiers before it count 0. The two entries of the first class also count the
  * reads with a strand whose longest occurrence run is 2, which keeps every reference with a posting,
- * on more than 64 postings and with a diagonal run: these are not handed on. */
+ * on more than 64 postings and with a diagonal run: these are not handed on. A batch of up to two
+ * reads per SM goes to the second class alone; the two entries are then that one's. */
 int mg_last_tier_counts(mg_index* ix, uint32_t* counts7);
 int mg_bucket_sizes(mg_index* ix, const uint32_t* hashes, uint32_t* counts, uint64_t n);
 

@@ -337,8 +337,7 @@ __global__ void __launch_bounds__(Warps * 32) k_classify_dual_list(DevIndex ix, 
 
 // Long-read tier over the dual tiers' leftovers and the plain form's, a block per read with work
 // stealing (the next read is taken while this one is classified), in two classes: LongSmem, then RestSmem
-// over what that leaves (its launch costs a batch without such reads 2.5 us), whose own leftovers go to the
-// global-memory tier.
+// over what that leaves, whose own leftovers go to the global-memory tier.
 template <class SM, int MinBlocks>
 __global__ void __launch_bounds__(2 * SM::H, MinBlocks) k_classify_long(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd,
                                                                      const uint32_t* list, const unsigned* list_n,
@@ -382,9 +381,9 @@ __global__ void __launch_bounds__(2 * PlainSmem::H) k_classify_plain(const __gri
   }
 }
 
-// Block and global tiers over a list of reads; the reads that do not fit go to the next list, or,
-// from the last tier, are marked for the oversize tier (kErrHuge: the host then runs the batch again
-// with it).
+// Block and global tiers over a list of reads (the kernel that fills it may still run when this one is
+// set up); the reads that do not fit go to the next list, or, from the last tier, are marked for the
+// oversize tier (kErrHuge: the host then runs the batch again with it).
 template <int G>
 __global__ void __launch_bounds__(G) k_classify_block(const __grid_constant__ DevIndex ix, BatchDev b, StageDev sd, const uint32_t* list,
                                                        const unsigned* list_n, unsigned* cursor, uint32_t* next,
@@ -395,6 +394,7 @@ __global__ void __launch_bounds__(G) k_classify_block(const __grid_constant__ De
   uint8_t* base = gws ? gws + (size_t)blockIdx.x * lay.total : dsm;
   const StrandWS ws = ws_from(base, lay, caps.c);
   RedTmp<G>* red = (RedTmp<G>*)(base + lay.red);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t n = *list_n;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(cursor, 1u);
@@ -1253,17 +1253,36 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
       if (tm) CU(cudaEventRecord(ix->ev[2], s));
       if (tm) CU(cudaEventRecord(ix->ev[3], s));
       if (ix->dix.n_refs <= (1u << 21)) {
-        k_classify_long<LongSmem, 4><<<grid(sh.long_blocks_per_sm * sms, 1), 2 * LongSmem::H, sizeof(LongSmem), s>>>(
-            ix->dix, b, sd, b.ovf0b, b.n_ovf0b, work_long, rest, n_rest, n_small, n_large);
+        // a batch of no more reads than the second class has blocks goes to it alone: it takes what the first
+        // takes, and the launch counts (16 reads of 75-300 bases: 45.6 us, 52.5 us with both; 16 of 1-20 kb:
+        // 91.6 us, 94.6 us on the first class alone)
+        const bool few = n <= 2u * (unsigned)sms;
+        if (!few)
+          k_classify_long<LongSmem, 4><<<grid(sh.long_blocks_per_sm * sms, 1), 2 * LongSmem::H, sizeof(LongSmem), s>>>(
+              ix->dix, b, sd, b.ovf0b, b.n_ovf0b, work_long, rest, n_rest, n_small, n_large);
         k_classify_long<RestSmem, 2><<<grid(2 * sms, 1), 2 * RestSmem::H, sizeof(RestSmem), s>>>(
-            ix->dix, b, sd, rest, n_rest, work_rest, b.ovf2, b.n_ovf2, nullptr, nullptr);
+            ix->dix, b, sd, few ? b.ovf0b : rest, few ? b.n_ovf0b : n_rest, work_rest, b.ovf2, b.n_ovf2,
+            few ? n_small : nullptr, few ? n_large : nullptr);
       } else {
         k_classify_block<kB2Threads><<<grid(sms, 1), kB2Threads, l2.total, s>>>(
             ix->dix, b, sd, b.ovf0b, b.n_ovf0b, b.work2, b.ovf2, b.n_ovf2, nullptr, l2, c2, 0);
       }
       if (tm) CU(cudaEventRecord(ix->ev[4], s));
-      k_classify_block<kB3Threads><<<grid(kB3Blocks, 1), kB3Threads, 0, s>>>(ix->dix, b, sd, b.ovf2, b.n_ovf2, b.work3, ovf3,
-                                                                    n_ovf3, w.gws.as<uint8_t>(), l3, c3, !w.hmode);
+      // set up while the kernel before it still runs (it waits for that kernel's end itself): the two that a
+      // batch without such reads passes through for nothing then take it no longer than one did (20,011 reads
+      // of 75-300 bases: 96.5 us without, 91.5 us so; with one kernel less 90.5 us). The same on the kernel
+      // before it costs some sizes more than it gives others (10,000 reads: 75 us without, 79 us so)
+      cudaLaunchConfig_t g = {};
+      g.gridDim = dim3(grid(kB3Blocks, 1));
+      g.blockDim = dim3(kB3Threads);
+      g.stream = s;
+      cudaLaunchAttribute early;
+      early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      early.val.programmaticStreamSerializationAllowed = 1;
+      g.attrs = &early;
+      g.numAttrs = 1;
+      CU(cudaLaunchKernelEx(&g, k_classify_block<kB3Threads>, ix->dix, b, sd, (const uint32_t*)b.ovf2, (const unsigned*)b.n_ovf2,
+                            b.work3, ovf3, n_ovf3, w.gws.as<uint8_t>(), l3, c3, (int)!w.hmode));
       // the oversize tier, once a batch of this workspace has needed it: one block while it has
       // no workspace (it only sizes the reads it gets)
       if (w.hmode)

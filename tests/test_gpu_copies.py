@@ -31,7 +31,16 @@ def _check(gix, oix, seqs, form="batched"):
     r = gix.classify(data, offs, form=form)
     d = diff(canon_from_gpu(r), canon_from_dump(oix.classify(data, offs, threads=os.cpu_count() or 1)))
     assert not d, "\n".join(d)
-    return r, gix.last_tier_counts()
+    c = gix.last_tier_counts()
+    if form == "batched":  # the same reads in a batch that both classes of the long-read tier share
+        reps = 300 // len(seqs) + 1
+        big = gix.classify(np.tile(data, reps), np.append(0, np.cumsum(np.tile(np.diff(offs), reps))).astype(np.uint64))
+        for f in r.reads.dtype.names:
+            if f != "cand_off":
+                assert np.array_equal(big.reads[f], np.tile(r.reads[f], reps)), f
+        assert np.array_equal(big.cands.view(np.uint8), np.tile(r.cands, reps).view(np.uint8))
+        assert gix.last_tier_counts()["block"] == reps * c["block"]
+    return r, c
 
 
 def _copies(rng, copies, n_refs, ref_len, seg_len, n_segs):

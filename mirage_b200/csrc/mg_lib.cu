@@ -1305,7 +1305,9 @@ int run_pipeline(mg_index* ix, Workspace& w, uint64_t n, const uint64_t* d_offs,
       // tiers of 64, 128 and 256 postings per strand, each over the one before's leftovers. The last
       // runs only for indexes whose reads start beyond the first (their strands' random hits fill the
       // smaller ones); elsewhere a strand of more than 128 postings lies in repeats, and the long-read
-      // tier takes it (200,000 reads of 250 bases, 16,000 such: 2.08 ms with it, 1.97 ms without)
+      // tier takes it. 200,000 reads of 250 bases inside segments of 8, 14 and 36 copies: 6.3, 7.0 and
+      // 10.4 ms so, 7.3, 8.3 and 10.8 ms with the 256-posting tier between; half on the flanks of segments
+      // of 14, 20 and 36 copies: 1.5, 3.1 and 5.5 ms so, 1.1, 1.5 and 3.8 ms with it
       // a small batch is spread over the warps, a read each if it can be (a chunk per warp waits for its
       // reads in turn: 16 reads 20 us in four chunks, 6 us so)
       const unsigned dual_warps = sh.dual_blocks_per_sm * sms * kW1Warps;

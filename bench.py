@@ -170,16 +170,21 @@ def seed_hashes(data: np.ndarray, offs: np.ndarray, k: int = 31, chunk_seeds: in
 
 def algorithmic_bytes(ix, reads, n_cands: int, k: int = 31) -> dict:
     """Bytes the path must move per batch (each term one access a minimal implementation
-    cannot avoid): the read bytes; per seed of both strands one 32-byte directory sector and the
-    32-byte sectors holding its postings (8 bytes each); per scored candidate two 32-byte
-    reference windows (head and tail of at least one run); 16 bytes of result per read and per
-    candidate."""
+    cannot avoid): the read bytes; per seed of both strands one 32-byte sector of the directory, or of
+    its hash slot when the index has them ("directory"), and the 32-byte sectors holding its postings
+    beyond ("postings": 8 bytes each; a slot's first sector holds three, its second four more); per
+    scored candidate two 32-byte reference windows (head and tail of at least one run); 16 bytes of
+    result per read and per candidate."""
     lens = reads.lengths().astype(np.int64)
+    slots = ix.info()["probe_slots"]
     post_bytes = 0
     n_seeds = 0
     for hs in seed_hashes(reads.data, reads.offs, k):
         cnt = ix.bucket_sizes(hs).astype(np.int64)
         n_seeds += len(hs)
+        if slots:
+            post_bytes += 32 * int((cnt > 3).sum())
+            cnt = np.maximum(cnt - 7, 0)
         post_bytes += int((((cnt * 8) + 31) // 32 * 32).sum())
     seed_bytes = 32 * n_seeds
     read_bytes = int(lens.sum())
@@ -637,12 +642,12 @@ def main():
                 "traffic": DUAL_TRAFFIC_DEFAULT if default_run else None,
                 "traffic_what": DUAL_TRAFFIC_WHAT if default_run else None,
                 "gather_peak": gather, "frac_of_gather": achieved / gather,
-                # the probe's own bytes (directory sectors + posting sectors) over the same time
+                # the probe's own bytes (directory or slot sectors + posting sectors) over the same time
                 "probe_frac_of_gather": (ab["directory"] + ab["postings"]) / (warp_ms / 1000) / 1e9 / gather,
                 "gather_peak_what": "random 32-byte sector gathers, 8 lanes per sector, over a 4 GiB buffer "
                                     "(mg_gather_bandwidth), measured in this run",
-                "kernel": "classification: k_classify_dual + k_finish_dual, beside them the general, block "
-                          "and global tiers (device step less compaction)",
+                "kernel": "classification: k_classify_dual + k_finish_dual, beside them the long-read and "
+                          "global tiers (device step less compaction)",
                 "kernel_ms": warp_ms,
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if hbm else "fallback 6650 GB/s",
                 "algorithmic_bytes_per_launch": ab}
@@ -685,11 +690,10 @@ def main():
                 "batched_over_plain_e2e": e2e / plain,
                 "served": served,
                 "kernel_ms_per_step": {"what": "dual tier with its finishing pass on the call's stream; the "
-                                               "general, block and global tiers on a second stream from the dual "
+                                               "long-read and global tiers on a second stream from the dual "
                                                "kernel's end, beside the finishing pass",
                                        "dual_warp_tier": kernel_ms[0] / args.steps,
-                                       "general_warp_tier": kernel_ms[1] / args.steps,
-                                       "block_tier": kernel_ms[2] / args.steps,
+                                       "long_read_tier": kernel_ms[2] / args.steps,
                                        "global_tier": kernel_ms[3] / args.steps,
                                        "compaction": kernel_ms[4] / args.steps},
                 "roofline": roof, "cpu_baseline": cpu, "parity": parity, "clocks": clk.summary(),

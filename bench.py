@@ -54,7 +54,7 @@ LAUNCHES_PER_BATCH = 8
 # default workload (1,000,000 reads, scale 1.0): a constant from one ncu capture of this kernel,
 # not a measurement of this run
 # dram__bytes_read.sum + dram__bytes_write.sum of k_classify_dual and of k_finish_dual, one launch each
-DUAL_TRAFFIC_DEFAULT = (2_986_232_832 + 47_951_616) + (357_686_528 + 63_106_304)
+DUAL_TRAFFIC_DEFAULT = (2_986_505_472 + 47_836_672) + (352_455_168 + 29_821_440)
 DUAL_TRAFFIC_WHAT = ("DRAM bytes per step of k_classify_dual + k_finish_dual (the kernels of kernel_ms but the "
                      "side tiers): a constant from one ncu capture of each on this workload "
                      "(dram__bytes_read.sum + dram__bytes_write.sum), not measured in this run")

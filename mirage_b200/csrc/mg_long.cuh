@@ -29,11 +29,11 @@
 //                      triangle and covered bases to its reference's sums and bitmap (MatrixCPU.cpp:18-214)
 //
 // What bounds it: latency, of the slots' DRAM pages and of some twenty group-wide steps a strand, with
-// eight strands in flight per SM (issue slots 27% used, DRAM 1.3 TB/s). Measured on a B200 against the
-// form before it (two sizes of block, one strand at a time on 256 threads, a hash set of (refID, found
+// eight strands in flight per SM (10,000 reads of 1-20 kb: issue slots 37% used, DRAM 1.7 TB/s; the
+// barriers hold the warps longest). Measured on a B200 against the form before it (two sizes of block, one strand at a time on 256 threads, a hash set of (refID, found
 // index) pairs, then a block per SM with two full sorts for what they left): 20,000 reads of 1-20 kb
-// on 5,000 references 5.86 -> 1.72 ms, 200,000 reads of 250 bases on references sharing repeats (36
-// copies of a segment) 4.50 -> 2.06 ms, 4,001 reads of 75 bases to 20 kb from host memory 1.28 -> 0.70 ms.
+// on 5,000 references 5.86 -> 1.66 ms, 200,000 reads of 250 bases on references sharing repeats (36
+// copies of a segment) 4.50 -> 1.69 ms, 4,001 reads of 75 bases to 20 kb from host memory 1.28 -> 0.65 ms.
 #pragma once
 #include "mg_lean.cuh"
 

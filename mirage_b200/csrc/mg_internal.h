@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <initializer_list>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -53,15 +54,27 @@ struct DevBuf {
   }
 };
 
-// A piece of a device buffer, by its offset.
+// A piece of a device buffer.
 struct DevPiece {
   uint8_t* p = nullptr;
-  uint64_t at = 0;
   template <class T>
   T* as() const {
     return (T*)p;
   }
 };
+// One allocation, or a kept one that is large enough, for pieces of the given bytes, each on a 256-byte
+// boundary.
+inline int alloc_pieces(DevBuf& buf, std::initializer_list<std::pair<DevPiece*, uint64_t>> pieces) {
+  uint64_t need = 0;
+  for (const auto& x : pieces) need += (x.second / 256 + 1) * 256;
+  if (buf.alloc(need)) return -1;
+  uint8_t* at = buf.as<uint8_t>();
+  for (const auto& x : pieces) {
+    x.first->p = at;
+    at += (x.second / 256 + 1) * 256;
+  }
+  return 0;
+}
 
 // Device buffers of one classification call in flight (a call owns one at a time).
 struct Workspace {

@@ -2119,25 +2119,11 @@ int mg_score_candidates(mg_index* ix, uint64_t n_strands, const uint64_t* q_off,
   // allocations on every call took half of it and more (20,000 strands with 27,000 candidates: 1.6 ms, on
   // some calls 4.9 ms; 0.69 ms now).
   DevPiece dq, db, dr, drun, dcs, dro, dsc, dpc, drl, dhit, derr;
-  uint64_t need = 0;
-  auto piece = [&](DevPiece& v, uint64_t bytes) {
-    v.at = need;
-    need += (bytes + 255) / 256 * 256;
-  };
-  piece(dq, (n_strands + 1) * 8);
-  piece(db, nb + 16);
-  piece(dr, nc * 4 + 4);
-  piece(drun, nr * 16 + 16);
-  piece(dcs, nc * 8 + 8);
-  piece(dro, (nc + 1) * 8);
-  piece(dsc, nc * 4 + 4);
-  piece(dpc, nc * 4 + 4);
-  piece(drl, nc * 4 + 4);
-  piece(dhit, nc * hw * 4 + 4);
-  piece(derr, 4);
-  if (ix->score_ws.alloc(need)) return set_error(MG_ERR_OOM, "scoring buffers");
-  for (DevPiece* v : {&dq, &db, &dr, &drun, &dcs, &dro, &dsc, &dpc, &drl, &dhit, &derr})
-    v->p = ix->score_ws.as<uint8_t>() + v->at;
+  if (alloc_pieces(ix->score_ws, {{&dq, (n_strands + 1) * 8}, {&db, nb + 16}, {&dr, nc * 4 + 4},
+                                  {&drun, nr * 16 + 16}, {&dcs, nc * 8 + 8}, {&dro, (nc + 1) * 8},
+                                  {&dsc, nc * 4 + 4}, {&dpc, nc * 4 + 4}, {&drl, nc * 4 + 4},
+                                  {&dhit, nc * hw * 4 + 4}, {&derr, 4}}))
+    return set_error(MG_ERR_OOM, "scoring buffers");
   cudaStream_t st = ix->stream;
   CU(cudaMemcpyAsync(dq.p, q_off, (n_strands + 1) * 8, cudaMemcpyHostToDevice, st));
   if (nb) CU(cudaMemcpyAsync(db.p, bases, nb, cudaMemcpyHostToDevice, st));

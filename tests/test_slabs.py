@@ -48,9 +48,10 @@ def test_oversize_reads_with_memory_for_few_workspaces():
     one = np.array([0, lens[0]], np.uint64)
     tight.classify(data[:lens[0]], one)  # and one workspace
     torch.cuda.empty_cache()
-    free = torch.cuda.mem_get_info(0)[0]
-    held = torch.empty(free - (72 << 20), dtype=torch.uint8, device="cuda:0")
+    held = []
     try:
+        while (spare := torch.cuda.mem_get_info(0)[0] - (72 << 20)) > (4 << 20):
+            held.append(torch.empty(min(spare, 16 << 30), dtype=torch.uint8, device="cuda:0"))
         got = [tight.classify(data, roffs) for _ in range(2)]
     finally:
         del held
